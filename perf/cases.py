@@ -59,7 +59,7 @@ def listed():
         # a new operator every call: assembly, change of basis, solver set-up, solve (changing coefficients)
         dict(name="new system 3d p2 32^3", kind="new", nx=32, ny=32, nz=32, p=2, variance=0.5),
         # independent systems solved from one graph launch
-        dict(name="batch of 6, 16^3 p2", kind="batch", count=6, n=16, p=2, variance=0.5),
+        dict(name="batch of 6 16^3 p2", kind="batch", count=6, n=16, p=2, variance=0.5),
     ]
 
 
