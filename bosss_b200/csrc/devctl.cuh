@@ -14,7 +14,7 @@
 namespace bsgpu {
 
 // Bits of the device error word of a captured solve (read by the host after the graph).
-enum { kDevErrNaN = 1, kDevErrResidualIncrease = 2, kDevErrSlots = 4, kDevErrKrylovNaN = 8 };
+enum { kDevErrNaN = 1, kDevErrResidualIncrease = 2, kDevErrSlots = 4, kDevErrKrylovNaN = 8, kDevErrWait = 16 };
 
 // Device state of one OrthonormalizationMultigrid level (CoreOrthonormalizationProcedure + loop).
 struct OrthoState {

@@ -1,0 +1,1019 @@
+// Persistent conjugate gradients (see pcg.cuh).
+#include <algorithm>
+#include <type_traits>
+
+#include "ldst.cuh"
+#include "packets.cuh"
+#include "pcg.cuh"
+
+namespace bsgpu {
+
+namespace {
+
+constexpr int kThreads = 256;       // large systems
+constexpr int kThreadsOne = 512;    // one tile per CTA: fewer arrivals at the barrier
+
+// Vectors that other SMs write during the kernel are read from L2.
+template <typename T, int V>
+__device__ __forceinline__ Vec<T, V> ldv_cg(const T* ptr) {
+  Vec<T, V> v;
+  if constexpr (sizeof(T) * V == 16) {
+    if constexpr (sizeof(T) == 8) {
+      const double2 d = __ldcg(reinterpret_cast<const double2*>(ptr));
+      v.a[0] = d.x; v.a[1] = d.y;
+    } else {
+      const float4 d = __ldcg(reinterpret_cast<const float4*>(ptr));
+      v.a[0] = d.x; v.a[1] = d.y; v.a[2] = d.z; v.a[3] = d.w;
+    }
+  } else if constexpr (sizeof(T) == 4 && V == 2) {
+    const float2 d = __ldcg(reinterpret_cast<const float2*>(ptr));
+    v.a[0] = d.x; v.a[1] = d.y;
+  } else {
+#pragma unroll
+    for (int q = 0; q < V; ++q) v.a[q] = __ldcg(ptr + q);
+  }
+  return v;
+}
+
+// A vector in plain memory.
+template <typename T, int V>
+struct PlainVec {
+  const T* x;
+  template <int NV>
+  __device__ __forceinline__ void load(int64_t idx, Vec<T, V> (&out)[NV]) const {
+#pragma unroll
+    for (int c = 0; c < NV; ++c) out[c] = ldv_cg<T, V>(x + idx + c * V);
+  }
+};
+
+// A vector of packets at epoch `ep`.
+template <typename T, int V>
+struct PacketVec {
+  const uint64_t* w;
+  unsigned ep;
+  unsigned int* fail;
+  static constexpr int WPV = sizeof(T) / 4;  // words per value
+  template <int NV>
+  __device__ __forceinline__ void load(int64_t idx, Vec<T, V> (&out)[NV]) const {
+    constexpr int NW = NV * V * WPV;
+    const uint64_t* p = w + idx * WPV;
+    uint64_t q[NW];
+    unsigned n = 0;
+    while (true) {
+      if constexpr (NW % 2 == 0 && (V * WPV) % 2 == 0) {
+#pragma unroll
+        for (int k = 0; k < NW; k += 2) ld_words(p + k, q[k], q[k + 1]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < NW; ++k) q[k] = ld_word(p + k);
+      }
+      bool ready = true;
+#pragma unroll
+      for (int k = 0; k < NW; ++k) ready = ready && packet_is(q[k], ep);
+      if (ready || spin_over(n, fail)) break;
+    }
+#pragma unroll
+    for (int c = 0; c < NV; ++c)
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        if constexpr (WPV == 2)
+          out[c].a[v] = packet_double(q[(c * V + v) * 2], q[(c * V + v) * 2 + 1]);
+        else
+          out[c].a[v] = __uint_as_float((unsigned)q[c * V + v]);
+      }
+  }
+};
+
+// Matrix values: with one tile per CTA the CTA's blocks stay in L1 across the iterations (cached loads), otherwise
+// they stream past it.
+template <typename ST, int V, bool CACHED>
+__device__ __forceinline__ Vec<ST, V> ldv_value(const ST* ptr, uint64_t pol) {
+  if constexpr (CACHED && sizeof(ST) >= 4)
+    return ldv_cached<ST, V>(ptr);
+  else
+    return ldv_stream<ST, V>(ptr, pol);
+}
+
+// Block rows of a uniform matrix: SPLIT * NP threads per block row, thread (s, r) sums the blocks s, s + SPLIT, ...
+// of DOF row r; the partial sums meet in shared memory and the threads with s = 0 own the row.
+template <typename T, int NP, int V, int SPLIT, typename ST, int THREADS, int MINCTAS = 1>
+struct UniformRows {
+  using Value = T;
+  static constexpr int kV = V;
+  static constexpr int kT = THREADS;
+  [[maybe_unused]] static constexpr int kMinCtas = MINCTAS;
+  // blocks of 15 and 20 exchange the new residual through shared memory (24^3 p = 3 FP64: 74 us per iteration against
+  // 79 with every thread recomputing its block's residual); smaller ones recompute it (64^3 p = 1: 71 against 89)
+  [[maybe_unused]] static constexpr bool kExchange = NP >= 15;
+  static constexpr bool kCached = MINCTAS == 1;  // one tile per CTA
+  static constexpr int RT = NP * SPLIT;
+  static constexpr int BPC = THREADS / RT;
+  const int64_t* __restrict__ rp;
+  const int32_t* __restrict__ ci;
+  const ST* __restrict__ vals;
+  int64_t nb;
+  // per tile
+  int64_t i, g;
+  int r, s, lb;
+  bool valid, own;
+  uint64_t pol;
+  __device__ __forceinline__ int64_t tiles() const { return (nb + BPC - 1) / BPC; }
+  __device__ __forceinline__ int64_t size() const { return nb * NP; }
+  // z_g = (D w)_g with w = r - alpha q of the row's block (q null: w = r); *wn: w of the row itself
+  __device__ __forceinline__ T precondition(const T* __restrict__ dinv, const T* rv, const T* qv, double alpha,
+                                            int64_t row, T* wn) const {
+    const int64_t blk = row / NP;
+    const int k = (int)(row - blk * NP);
+    if (dinv == nullptr) {
+      const T rr = __ldcg(rv + row);
+      return *wn = qv != nullptr ? (T)((double)rr - alpha * (double)__ldcg(qv + row)) : rr;
+    }
+    const T* D = dinv + blk * (NP * NP) + k;
+    T z = 0, own_w = 0;
+#pragma unroll
+    for (int c = 0; c < NP / V; ++c) {
+      const Vec<T, V> a = ldv_cg<T, V>(rv + blk * NP + c * V);
+      Vec<T, V> b{};
+      if (qv != nullptr) b = ldv_cg<T, V>(qv + blk * NP + c * V);
+#pragma unroll
+      for (int u = 0; u < V; ++u) {
+        const T w = qv != nullptr ? (T)((double)a.a[u] - alpha * (double)b.a[u]) : a.a[u];
+        z = fma(__ldg(D + (c * V + u) * NP), w, z);
+        if (c * V + u == k) own_w = w;
+      }
+    }
+    *wn = own_w;
+    return z;
+  }
+  __device__ __forceinline__ void begin() {
+    const int t = threadIdx.x;
+    lb = t / RT;
+    const int u = t - lb * RT;
+    s = u / NP;
+    r = u - s * NP;
+    pol = policy_evict_first();
+  }
+  __device__ __forceinline__ void at(int64_t tile) {
+    i = tile * BPC + lb;
+    valid = (lb < BPC) && (i < nb);
+    own = valid && s == 0;
+    g = i * NP + r;
+  }
+  // the operand is loaded in groups of NV chunks (with packets a group is one wait)
+  static constexpr int NC = NP / V;
+  static constexpr int kGroup = !kCached ? 1 : (sizeof(T) == 8 ? 6 : 12) / V;
+  static constexpr int NV = NC < kGroup ? NC : kGroup;
+  template <int M, class Vector>
+  __device__ __forceinline__ void group(const Vector& x, const ST* vb, int64_t x0, int h, T& acc0, T& acc1) const {
+    Vec<T, V> xv[M];
+    Vec<ST, V> av[M];
+#pragma unroll
+    for (int c = 0; c < M; ++c) av[c] = ldv_value<ST, V, kCached>(vb + (h + c) * (NP * V), pol);
+    x.load(x0 + h * V, xv);
+#pragma unroll
+    for (int c = 0; c < M; ++c) {
+#pragma unroll
+      for (int q = 0; q < V; ++q) {
+        if (((h + c) * V + q) & 1)
+          acc1 = fma(widen<T>(av[c].a[q]), xv[c].a[q], acc1);
+        else
+          acc0 = fma(widen<T>(av[c].a[q]), xv[c].a[q], acc0);
+      }
+    }
+  }
+  template <class Vector>
+  __device__ __forceinline__ T product(const Vector& x, T* sm) {
+    T acc0 = 0, acc1 = 0;
+    if (valid) {
+      const int64_t k1 = __ldg(rp + i + 1);
+      for (int64_t k = __ldg(rp + i) + s; k < k1; k += SPLIT) {
+        const int64_t x0 = (int64_t)__ldg(ci + k) * NP;
+        const ST* vb = vals + k * (NP * NP) + r * V;
+#pragma unroll
+        for (int h = 0; h + NV <= NC; h += NV) group<NV>(x, vb, x0, h, acc0, acc1);
+        if constexpr (NC % NV != 0) group<NC % NV>(x, vb, x0, NC - NC % NV, acc0, acc1);
+      }
+    }
+    T acc = acc0 + acc1;
+    if constexpr (SPLIT > 1) {
+      sm[threadIdx.x] = acc;
+      __syncthreads();
+      if (own) {
+#pragma unroll
+        for (int q = 1; q < SPLIT; ++q) acc += sm[threadIdx.x + q * NP];
+      }
+      __syncthreads();
+    }
+    return acc;
+  }
+  // z = D rn for the owner's row (D column-major per block), rn given by the owners
+  __device__ __forceinline__ T solve(const T* __restrict__ dinv, T rn, T* sm) {
+    if (own) sm[lb * NP + r] = rn;
+    __syncthreads();
+    T z = 0;
+    if (valid) {
+      const T* D = dinv + i * (NP * NP) + r;
+      const T* rb = sm + lb * NP;
+#pragma unroll
+      for (int c0 = 0; c0 < NP; c0 += SPLIT) {
+        const int c = c0 + s;
+        if (c < NP) z = fma(__ldg(D + c * NP), rb[c], z);
+      }
+    }
+    __syncthreads();
+    if constexpr (SPLIT > 1) {
+      sm[threadIdx.x] = z;
+      __syncthreads();
+      if (own) {
+#pragma unroll
+        for (int q = 1; q < SPLIT; ++q) z += sm[threadIdx.x + q * NP];
+      }
+      __syncthreads();
+    }
+    return z;
+  }
+};
+
+// Any block sizes: a tile is a pack of whole block rows (at most 256 DOF rows); SPLIT threads per DOF row as above.
+template <typename T, int V, int SPLIT, typename ST, bool ONE>
+struct GeneralRows {
+  using Value = T;
+  static constexpr int kRows = 256;
+  static constexpr int kV = V;
+  static constexpr int kT = kRows * SPLIT;
+  static constexpr int kMinCtas = ONE ? 1 : 4;
+  static constexpr bool kExchange = false;
+  const int64_t* __restrict__ rp;
+  const int32_t* __restrict__ ci;
+  const int32_t* __restrict__ len;
+  const int64_t* __restrict__ i0;
+  const int64_t* __restrict__ boff;
+  const int32_t* __restrict__ row2blk;
+  const int64_t* __restrict__ cta_row0;
+  const int64_t* __restrict__ doff;
+  const ST* __restrict__ vals;
+  int64_t ncta, n;
+  int64_t i, g, row0;
+  int r, I, s, l;
+  bool valid, own;
+  uint64_t pol;
+  __device__ __forceinline__ int64_t tiles() const { return ncta; }
+  __device__ __forceinline__ int64_t size() const { return n; }
+  __device__ __forceinline__ T precondition(const T* __restrict__ dinv, const T* rv, const T* qv, double alpha,
+                                            int64_t row, T* wn) const {
+    const T rr = __ldcg(rv + row);
+    *wn = qv != nullptr ? (T)((double)rr - alpha * (double)__ldcg(qv + row)) : rr;
+    if (dinv == nullptr) return *wn;
+    const int64_t blk = __ldg(row2blk + row), b0 = __ldg(i0 + blk);
+    const int len_b = __ldg(len + blk);
+    const T* D = dinv + __ldg(doff + blk) + (row - b0);
+    T z = 0;
+    for (int c = 0; c < len_b; ++c) {
+      const T a = __ldcg(rv + b0 + c);
+      const T w = qv != nullptr ? (T)((double)a - alpha * (double)__ldcg(qv + b0 + c)) : a;
+      z = fma(__ldg(D + (int64_t)c * len_b), w, z);
+    }
+    return z;
+  }
+  __device__ __forceinline__ void begin() {
+    pol = policy_evict_first();
+    s = threadIdx.x / kRows;
+    l = threadIdx.x - s * kRows;
+  }
+  __device__ __forceinline__ void at(int64_t tile) {
+    row0 = __ldg(cta_row0 + tile);
+    g = row0 + l;
+    valid = g < __ldg(cta_row0 + tile + 1);
+    own = valid && s == 0;
+    i = valid ? __ldg(row2blk + g) : 0;
+    r = valid ? (int)(g - __ldg(i0 + i)) : 0;
+    I = valid ? __ldg(len + i) : 0;
+  }
+  template <class Vector>
+  __device__ __forceinline__ T product(const Vector& x, T* sm) {
+    T acc = 0;
+    if (valid) {
+      const int64_t k1 = __ldg(rp + i + 1);
+      for (int64_t k = __ldg(rp + i) + s; k < k1; k += SPLIT) {
+        const int64_t j = __ldg(ci + k);
+        const int J = __ldg(len + j);
+        const ST* vb = vals + __ldg(boff + k) + r * V;
+        const int64_t x0 = __ldg(i0 + j);
+        int c = 0;
+        for (; c + 2 * V <= J; c += 2 * V) {
+          Vec<T, V> xv[2];
+          const Vec<ST, V> a = ldv_value<ST, V, ONE>(vb + (int64_t)(c / V) * I * V, pol);
+          const Vec<ST, V> b = ldv_value<ST, V, ONE>(vb + (int64_t)(c / V + 1) * I * V, pol);
+          x.load(x0 + c, xv);
+#pragma unroll
+          for (int q = 0; q < V; ++q) acc = fma(widen<T>(a.a[q]), xv[0].a[q], acc);
+#pragma unroll
+          for (int q = 0; q < V; ++q) acc = fma(widen<T>(b.a[q]), xv[1].a[q], acc);
+        }
+        for (; c < J; c += V) {
+          Vec<T, V> xv[1];
+          const Vec<ST, V> a = ldv_value<ST, V, ONE>(vb + (int64_t)(c / V) * I * V, pol);
+          x.load(x0 + c, xv);
+#pragma unroll
+          for (int q = 0; q < V; ++q) acc = fma(widen<T>(a.a[q]), xv[0].a[q], acc);
+        }
+      }
+    }
+    return sum_split(acc, sm);
+  }
+  // the owner's sum of its row's SPLIT partial values
+  __device__ __forceinline__ T sum_split(T v, T* sm) {
+    if constexpr (SPLIT > 1) {
+      sm[threadIdx.x] = v;
+      __syncthreads();
+      if (own) {
+#pragma unroll
+        for (int q = 1; q < SPLIT; ++q) v += sm[threadIdx.x + q * kRows];
+      }
+      __syncthreads();
+    }
+    return v;
+  }
+  __device__ __forceinline__ T solve(const T* __restrict__ dinv, T rn, T* sm) {
+    if (own) sm[l] = rn;
+    __syncthreads();
+    T z = 0;
+    if (valid) {
+      const T* D = dinv + __ldg(doff + i) + r;
+      const T* rb = sm + (g - r - row0);
+      for (int c = s; c < I; c += SPLIT) z = fma(__ldg(D + (int64_t)c * I), rb[c], z);
+    }
+    __syncthreads();
+    return sum_split(z, sm);
+  }
+};
+
+// Barrier of the first THREADS threads of the CTA (the streaming kernel has a further warp that does not take part).
+template <int THREADS>
+__device__ __forceinline__ void sync_threads() {
+  asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+}
+
+// The CTA's sums of K accumulators, in the lanes of warp 0.
+template <int K, int THREADS>
+__device__ __forceinline__ void cta_sums(const double (&acc)[K], double (&out)[K], double (*red)[2]) {
+  constexpr int W = THREADS / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    double v = acc[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) red[warp][k] = v;
+  }
+  sync_threads<THREADS>();
+  if (warp == 0) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      double v = lane < W ? red[lane][k] : 0.0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      out[k] = v;
+    }
+  }
+}
+
+// ... written to partial[k * grid + cta] (the following barrier publishes them)
+template <int K, int THREADS>
+__device__ __forceinline__ void put_partials(const double (&acc)[K], double* __restrict__ partial, double (*red)[2]) {
+  double v[K];
+  cta_sums<K, THREADS>(acc, v, red);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) __stcg(partial + (int64_t)k * gridDim.x + blockIdx.x, v[k]);
+  }
+}
+
+// The grid's sums in a fixed order, the same value in every thread of every CTA.
+template <int K, int THREADS>
+__device__ __forceinline__ void grid_sums(double (&out)[K], const double* __restrict__ partial, double (*red)[2]) {
+  __shared__ double tot[2];
+  double acc[K], v[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    acc[k] = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += THREADS) acc[k] += __ldcg(partial + (int64_t)k * gridDim.x + b);
+  }
+  cta_sums<K, THREADS>(acc, v, red);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) tot[k] = v[k];
+  }
+  sync_threads<THREADS>();
+#pragma unroll
+  for (int k = 0; k < K; ++k) out[k] = tot[k];
+}
+
+// The same sums exchanged as packets (w: K values per CTA): no counter and no fence, the arrival of a CTA's packet is
+// its arrival at the reduction.  Warp 0 collects, four packets per lane in flight.
+template <int K, int THREADS>
+__device__ __forceinline__ bool exchange_sums(const double (&acc)[K], double (&out)[K], uint64_t* w, unsigned ep,
+                                              unsigned int* fail, double (*red)[2]) {
+  __shared__ double tot[2];
+  __shared__ int failed;
+  double v[K];
+  cta_sums<K, THREADS>(acc, v, red);
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    if (lane < K) {
+      double mine = v[0];
+      if (K > 1 && lane == 1) mine = v[K - 1];
+      put_packet(w + ((int64_t)blockIdx.x * K + lane) * 2, mine, ep);
+    }
+    const int G = gridDim.x;
+    double s[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) s[k] = 0.0;
+    unsigned n = 0;
+    bool over = false;
+    for (int b0 = lane; b0 < G; b0 += 128) {
+      uint64_t q[4][2 * K];
+      bool ready;
+      do {
+        ready = true;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (b0 + 32 * u < G) {
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+              ld_words(w + ((int64_t)(b0 + 32 * u) * K + k) * 2, q[u][2 * k], q[u][2 * k + 1]);
+          }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (b0 + 32 * u < G) {
+#pragma unroll
+            for (int k = 0; k < 2 * K; ++k) ready = ready && packet_is(q[u][k], ep);
+          }
+      } while (!ready && !(over = spin_over(n, fail)));
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (b0 + 32 * u < G) {
+#pragma unroll
+          for (int k = 0; k < K; ++k) s[k] += packet_double(q[u][2 * k], q[u][2 * k + 1]);
+        }
+    }
+    over = __any_sync(0xffffffffu, over);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+      if (lane == 0) tot[k] = s[k];
+    }
+    if (lane == 0) failed = over;
+  }
+  sync_threads<THREADS>();
+#pragma unroll
+  for (int k = 0; k < K; ++k) out[k] = tot[k];
+  return failed == 0;
+}
+
+// Grid barrier (all CTAs are resident: cooperative launch).  False when the bounded wait ran out somewhere.
+template <int THREADS>
+__device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int target) {
+  __shared__ int ok;
+  sync_threads<THREADS>();
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    unsigned int v = 0, n = 0, failed = 0;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      if (v >= target) break;
+      if ((++n & 1023u) == 0) {
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(failed) : "l"(bar + 1) : "memory");
+        if (n >= kSpinLimit) {
+          atomicExch(bar + 1, 1u);
+          failed = 1;
+        }
+      }
+    } while (!failed);
+    ok = !failed;
+  }
+  sync_threads<THREADS>();
+  return ok != 0;
+}
+
+// The scalar step after r.z and r.r are known (SoftPCG.cs:113-194 with IterativeSolverConfig's termination); the same
+// in every thread of the grid.
+struct CgScalars {
+  double rz, rr, rr0, it, beta, pq;
+  bool stop;
+  template <typename T>
+  __device__ __forceinline__ void begin(const PcgCall<T>& a, double rz_, double rr_) {
+    rz = rz_;
+    rr = rr0 = rr_;
+    it = beta = pq = 0.0;
+    stop = a.stop_nonfinite && !isfinite(sqrt(rr0));
+    terminate(a);
+  }
+  template <typename T>
+  __device__ __forceinline__ void resume(const PcgCall<T>& a) {
+    rz = a.s[0];
+    pq = a.s[1];
+    rr = a.s[3];
+    rr0 = a.s[4];
+    it = a.s[5];
+    beta = a.s[6];
+    stop = false;
+  }
+  template <typename T>
+  __device__ __forceinline__ void terminate(const PcgCall<T>& a) {
+    const double R = sqrt(rr), R0 = sqrt(rr0), eps = 2.2204460492503131e-16 * 1000;
+    if (it > a.min_iter) {
+      const bool done = (a.mode == 0) ? (R < R0 * a.tol + a.tol) : (R < R0 * a.tol);
+      if (done || it > a.max_iter || R < eps || R0 < eps) stop = true;
+    }
+  }
+  template <typename T>
+  __device__ __forceinline__ void step(const PcgCall<T>& a, double rz_new, double rr_new) {
+    beta = rz_new / rz;
+    rz = rz_new;
+    rr = rr_new;
+    it += 1.0;
+    terminate(a);
+    if (!isfinite(rz) || !isfinite(rr)) stop = true;
+    const long iter = (long)it;
+    if (a.hist != nullptr && blockIdx.x == 0 && threadIdx.x == 0 && (stop || iter % kPcgHistory == 0)) {
+      const long e = (iter + kPcgHistory - 1) / kPcgHistory - 1 - a.hist_base;
+      if (e >= 0 && e < a.hist_cap) a.hist[e] = sqrt(rr);
+    }
+  }
+  template <typename T>
+  __device__ __forceinline__ void end(const PcgCall<T>& a, bool ok) const {
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    a.s[0] = rz;
+    a.s[1] = pq;
+    a.s[2] = rz;
+    a.s[3] = rr;
+    a.s[4] = rr0;
+    a.s[5] = it;
+    a.s[6] = beta;
+    a.s[7] = !ok ? kPcgFailed : stop ? kPcgDone : kPcgRunning;
+    if (!ok && a.err != nullptr) atomicOr(a.err, a.err_bit);
+  }
+};
+
+// Large systems: tiles blockIdx.x, blockIdx.x + gridDim.x, ... of block rows for the products, one thread per DOF row
+// over the whole grid for the vectors, which live in memory; a counting barrier after each of the three phases of an
+// iteration.  With small blocks the vector phase recomputes the new residual of a whole block in each of the block's
+// threads (from the old one, two residual buffers) instead of exchanging it, and the scalars sit in shared memory, so
+// that no phase has a CTA barrier inside and the registers allow the occupancy that the stream of blocks needs.
+// Bound by HBM (or L2) traffic: 32^3 p = 1 FP64 (29 MB) 17 us per iteration (25 as four launches), 64^3 p = 1 (232 MB)
+// 71 us (74), 400^2 p = 1 (57 MB) 35 us (64).
+template <class Rows>
+__global__ void __launch_bounds__(Rows::kT, Rows::kMinCtas)
+    pcg_kernel(Rows rows, PcgCall<typename Rows::Value> a, typename Rows::Value* __restrict__ r2,
+               double* __restrict__ partial, unsigned int* __restrict__ bar) {
+  using T = typename Rows::Value;
+  constexpr int TH = Rows::kT, V = Rows::kV;
+  __shared__ T sm[TH];
+  __shared__ double red[TH / 32][2];
+  __shared__ CgScalars c;
+  if (!a.start && a.s[7] != kPcgRunning) return;
+  rows.begin();
+  const int64_t first = (int64_t)blockIdx.x * TH + threadIdx.x, stride = (int64_t)gridDim.x * TH;
+  unsigned int target = 0;
+  bool ok = true;
+  T* r_now = a.r;
+  T* r_next = r2;
+  if (a.start) {
+    if (a.zero) {
+      for (int64_t g = first; g < rows.size(); g += stride) {
+        a.x[g] = T(0);
+        a.r[g] = a.b[g];
+      }
+    } else {
+      for (int64_t tile = blockIdx.x; tile < rows.tiles(); tile += gridDim.x) {
+        rows.at(tile);
+        const T ax = rows.product(PlainVec<T, V>{a.x}, (T*)nullptr);
+        if (rows.own) a.r[rows.g] = a.b[rows.g] - ax;
+      }
+    }
+    ok = grid_barrier<TH>(bar, target += gridDim.x);
+    double acc[2] = {0.0, 0.0}, tot[2];
+    for (int64_t g = first; ok && g < rows.size(); g += stride) {
+      T w;
+      const T z = rows.precondition(a.dinv, a.r, (const T*)nullptr, 0.0, g, &w);
+      a.z[g] = z;
+      a.p[g] = z;
+      acc[0] = fma((double)w, (double)z, acc[0]);
+      acc[1] = fma((double)w, (double)w, acc[1]);
+    }
+    put_partials<2, TH>(acc, partial, red);
+    ok = grid_barrier<TH>(bar, target += gridDim.x) && ok;
+    grid_sums<2, TH>(tot, partial, red);
+    if (threadIdx.x == 0) c.begin(a, tot[0], tot[1]);
+  } else {
+    if (threadIdx.x == 0) c.resume(a);
+    ok = grid_barrier<TH>(bar, target += gridDim.x);  // everyone has read the scalars
+  }
+  sync_threads<TH>();
+  for (int n = 0; ok && !c.stop && n < a.cap; ++n) {
+    {  // q = A p, p.q
+      double acc[1] = {0.0}, tot[1];
+      for (int64_t tile = blockIdx.x; tile < rows.tiles(); tile += gridDim.x) {
+        rows.at(tile);
+        const T vq = rows.product(PlainVec<T, V>{a.p}, (T*)nullptr);
+        if (rows.own) {
+          a.q[rows.g] = vq;
+          acc[0] = fma((double)__ldcg(a.p + rows.g), (double)vq, acc[0]);
+        }
+      }
+      put_partials<1, TH>(acc, partial, red);
+      ok = grid_barrier<TH>(bar, target += gridDim.x);
+      if (!ok) break;
+      grid_sums<1, TH>(tot, partial, red);
+      if (threadIdx.x == 0) c.pq = tot[0];
+      sync_threads<TH>();
+    }
+    {  // x += alpha p, r -= alpha q, z = D r, r.z, r.r
+      const double alpha = c.rz / c.pq;
+      double acc[2] = {0.0, 0.0}, tot[2];
+      if constexpr (Rows::kExchange) {
+        for (int64_t tile = blockIdx.x; tile < rows.tiles(); tile += gridDim.x) {
+          rows.at(tile);
+          T w = 0;
+          if (rows.own) {
+            const T vp = __ldcg(a.p + rows.g), vq = __ldcg(a.q + rows.g);
+            const T vx = __ldcg(a.x + rows.g), vr = __ldcg(r_now + rows.g);
+            a.x[rows.g] = (T)((double)vx + alpha * (double)vp);
+            w = (T)((double)vr - alpha * (double)vq);
+            r_next[rows.g] = w;
+          }
+          const T z = a.dinv ? rows.solve(a.dinv, w, sm) : w;
+          if (rows.own) {
+            a.z[rows.g] = z;
+            acc[0] = fma((double)w, (double)z, acc[0]);
+            acc[1] = fma((double)w, (double)w, acc[1]);
+          }
+        }
+      } else {
+        for (int64_t g = first; g < rows.size(); g += stride) {
+          const T vp = __ldcg(a.p + g), vx = __ldcg(a.x + g);
+          T w;
+          const T z = rows.precondition(a.dinv, r_now, a.q, alpha, g, &w);
+          a.x[g] = (T)((double)vx + alpha * (double)vp);
+          r_next[g] = w;
+          a.z[g] = z;
+          acc[0] = fma((double)w, (double)z, acc[0]);
+          acc[1] = fma((double)w, (double)w, acc[1]);
+        }
+      }
+      T* const h = r_now;
+      r_now = r_next;
+      r_next = h;
+      put_partials<2, TH>(acc, partial, red);
+      ok = grid_barrier<TH>(bar, target += gridDim.x);
+      if (!ok) break;
+      grid_sums<2, TH>(tot, partial, red);
+      if (threadIdx.x == 0) c.step(a, tot[0], tot[1]);
+      sync_threads<TH>();
+    }
+    if (c.stop) break;
+    {
+      const double beta = c.beta;
+#pragma unroll 4
+      for (int64_t g = first; g < rows.size(); g += stride)  // p = z + beta p
+        a.p[g] = (T)((double)__ldcg(a.z + g) + beta * (double)__ldcg(a.p + g));
+    }
+    ok = grid_barrier<TH>(bar, target += gridDim.x);
+  }
+  if (threadIdx.x == 0 && atomicAdd(bar + 2, 1u) == gridDim.x - 1) {  // the last CTA leaves the barrier at zero
+    bar[0] = bar[1] = bar[2] = 0u;
+    __threadfence();
+  }
+  c.end(a, ok);
+}
+
+// One tile per CTA: the rows' x, r, z, p and q stay in registers and the CTA's blocks in L1 for the whole solve.  What
+// other CTAs need - the direction p and the partial sums - goes through packets, so an iteration waits three times
+// for one store to be seen (p by its neighbours' products, p.q, and r.z with r.r) and never for a counter.
+// Bound by the latency of those exchanges: 64^2 p = 2 FP64 (24,576 unknowns) 7.4 us per iteration, 21 as four launches
+// of a graph; 24^3 p = 0 7.7 us (32 as nine launches).
+// No packet is overwritten before everybody has read it: the p of the next epoch is stored after the exchange of
+// r.z, which every CTA enters after its product; a sum of the next epoch after an exchange that every CTA enters
+// after having read the sum before.
+template <class Rows>
+__global__ void __launch_bounds__(Rows::kT) pcg_small_kernel(Rows rows, PcgCall<typename Rows::Value> a,
+                                                             uint64_t* __restrict__ packets,
+                                                             unsigned int* __restrict__ state) {
+  using T = typename Rows::Value;
+  constexpr int TH = Rows::kT, V = Rows::kV;
+  constexpr int WPV = sizeof(T) / 4;
+  __shared__ T sm[TH];
+  __shared__ double red[TH / 32][2];
+  if (!a.start && a.s[7] != kPcgRunning) return;
+  uint64_t* const pq_packets = packets;                             // 2 words per CTA
+  uint64_t* const rz_packets = packets + 2 * (int64_t)gridDim.x;    // 4 words per CTA
+  uint64_t* const p_packets = packets + 6 * (int64_t)gridDim.x;     // the direction
+  unsigned int* const fail = state + 1;
+  unsigned ep = state[0];
+  bool ok = true;
+  CgScalars c{};
+  T vx = 0, vr = 0, vz = 0, vp = 0;
+  rows.begin();
+  rows.at(blockIdx.x);
+  if (a.start) {
+    T ax = 0;
+    if (!a.zero) ax = rows.product(PlainVec<T, V>{a.x}, sm);
+    if (rows.own) {
+      vx = a.zero ? T(0) : __ldcg(a.x + rows.g);
+      vr = a.zero ? a.b[rows.g] : a.b[rows.g] - ax;
+    }
+    vz = a.dinv ? rows.solve(a.dinv, vr, sm) : vr;
+    vp = vz;
+    ++ep;
+    double acc[2] = {0.0, 0.0}, tot[2];
+    if (rows.own) {
+      put_packet(p_packets + rows.g * WPV, vp, ep);
+      acc[0] = (double)vr * (double)vz;
+      acc[1] = (double)vr * (double)vr;
+    }
+    ok = exchange_sums<2, TH>(acc, tot, rz_packets, ep, fail, red);
+    c.begin(a, tot[0], tot[1]);
+  } else {
+    c.resume(a);
+    if (rows.own) {
+      vx = __ldcg(a.x + rows.g);
+      vr = __ldcg(a.r + rows.g);
+      vz = __ldcg(a.z + rows.g);
+      vp = __ldcg(a.p + rows.g);
+    }
+  }
+  for (int n = 0; ok && !c.stop && n < a.cap; ++n) {
+    const T vq = rows.product(PacketVec<T, V>{p_packets, ep, fail}, sm);
+    {
+      double acc[1] = {rows.own ? (double)vp * (double)vq : 0.0}, tot[1];
+      ok = exchange_sums<1, TH>(acc, tot, pq_packets, ep, fail, red);
+      if (!ok) break;
+      c.pq = tot[0];
+    }
+    {
+      const double alpha = c.rz / c.pq;
+      double acc[2] = {0.0, 0.0}, tot[2];
+      if (rows.own) {
+        vx = (T)((double)vx + alpha * (double)vp);
+        vr = (T)((double)vr - alpha * (double)vq);
+      }
+      vz = a.dinv ? rows.solve(a.dinv, vr, sm) : vr;
+      if (rows.own) {
+        acc[0] = (double)vr * (double)vz;
+        acc[1] = (double)vr * (double)vr;
+      }
+      ok = exchange_sums<2, TH>(acc, tot, rz_packets, ep + 1, fail, red);
+      if (!ok) break;
+      c.step(a, tot[0], tot[1]);
+    }
+    ++ep;
+    if (c.stop) break;
+    if (rows.own) {
+      vp = (T)((double)vz + c.beta * (double)vp);
+      put_packet(p_packets + rows.g * WPV, vp, ep);
+    }
+  }
+  if (rows.own) {
+    a.x[rows.g] = vx;
+    if (!c.stop) {
+      a.r[rows.g] = vr;
+      a.z[rows.g] = vz;
+      a.p[rows.g] = vp;
+    }
+  }
+  if (threadIdx.x == 0 && atomicAdd(state + 2, 1u) == gridDim.x - 1) {
+    state[0] = ok ? ep : ep + 8;  // beyond every epoch that a CTA can have reached
+    state[1] = state[2] = 0u;
+    __threadfence();
+  }
+  c.end(a, ok);
+}
+
+// ---- choice and launch ------------------------------------------------------------------------------------------
+
+template <class R>
+struct Tag { using Rows = R; };
+// f(block size, chunk width) for the uniform matrices with kernels of their own; false for the others
+template <typename T, typename ST, class F>
+bool pick_uniform(const Matrix& A, F&& f) {
+  if (!A.uniform) return false;
+#define BSGPU_PCG(NP, VV) \
+  if (A.Np == NP && A.V == VV) return f(std::integral_constant<int, NP>{}, std::integral_constant<int, VV>{});
+  if constexpr (sizeof(ST) == 2) {
+    BSGPU_PCG(4, 4) BSGPU_PCG(10, 2) BSGPU_PCG(20, 4)
+  } else {
+    BSGPU_PCG(1, 1) BSGPU_PCG(3, 1) BSGPU_PCG(6, 2) BSGPU_PCG(10, 2) BSGPU_PCG(15, 1)
+    if constexpr (sizeof(T) == 4) {
+      BSGPU_PCG(4, 4) BSGPU_PCG(20, 4)
+    } else {
+      BSGPU_PCG(4, 2) BSGPU_PCG(20, 2)
+    }
+  }
+#undef BSGPU_PCG
+  return false;
+}
+
+// Calls f(Tag<Rows>) with the Rows type of the small kernel; false where there is none.
+template <typename T, typename ST, class F>
+bool pick_small(const Matrix& A, int split, F&& f) {
+  if (pick_uniform<T, ST>(A, [&](auto np, auto v) {
+        constexpr int NP = decltype(np)::value, V = decltype(v)::value;
+        if (split == 4) return f(Tag<UniformRows<T, NP, V, 4, ST, kThreadsOne>>{});
+        if (split == 2) return f(Tag<UniformRows<T, NP, V, 2, ST, kThreadsOne>>{});
+        return f(Tag<UniformRows<T, NP, V, 1, ST, kThreadsOne>>{});
+      }))
+    return true;
+  if constexpr (sizeof(ST) != 2) {
+    auto general = [&](auto v) {
+      constexpr int V = decltype(v)::value;
+      if (split == 4) return false;
+      if (split == 2) return f(Tag<GeneralRows<T, V, 2, ST, true>>{});
+      return f(Tag<GeneralRows<T, V, 1, ST, true>>{});
+    };
+    if (A.uniform && pick_uniform<T, ST>(A, [](auto, auto) { return true; })) return false;
+    if (A.V == 1) return general(std::integral_constant<int, 1>{});
+    if (A.V == 2) return general(std::integral_constant<int, 2>{});
+    if constexpr (sizeof(T) == 4) {
+      if (A.V == 4) return general(std::integral_constant<int, 4>{});
+    }
+  }
+  return false;
+}
+
+// Calls f(Tag<Rows>) with the Rows type of the large kernel.
+template <typename T, typename ST, class F>
+bool pick_large(const Matrix& A, F&& f) {
+  if (pick_uniform<T, ST>(A, [&](auto np, auto v) {
+        constexpr int NP = decltype(np)::value, V = decltype(v)::value;
+        // CTAs per SM: 4 (64 registers); blocks of 10 stream better from 5.  At 32^3 p = 2 FP64 (179 MB) 55 us per
+        // iteration against 60, at 200^2 p = 4 (blocks of 15, 359 MB) 142 against 130.
+        constexpr int MINCTAS = NP == 10 ? 5 : 4;
+        return f(Tag<UniformRows<T, NP, V, 1, ST, kThreads, MINCTAS>>{});
+      }))
+    return true;
+  if constexpr (sizeof(ST) != 2) {
+    if (A.V == 1) return f(Tag<GeneralRows<T, 1, 1, ST, false>>{});
+    if (A.V == 2) return f(Tag<GeneralRows<T, 2, 1, ST, false>>{});
+    if constexpr (sizeof(T) == 4) {
+      if (A.V == 4) return f(Tag<GeneralRows<T, 4, 1, ST, false>>{});
+    }
+  }
+  return false;
+}
+
+template <class Rows>
+struct IsGeneral { static constexpr bool value = false; };
+template <typename T, int V, int SPLIT, typename ST, bool ONE>
+struct IsGeneral<GeneralRows<T, V, SPLIT, ST, ONE>> { static constexpr bool value = true; };
+
+template <class Rows>
+Rows rows_of(const Matrix& A, decltype(Rows::vals) vals) {
+  Rows rows{};
+  rows.rp = A.rp.p;
+  rows.ci = A.ci.p;
+  rows.vals = vals;
+  if constexpr (IsGeneral<Rows>::value) {
+    rows.len = A.len.p;
+    rows.i0 = A.i0.p;
+    rows.boff = A.boff.p;
+    rows.row2blk = A.row2blk.p;
+    rows.cta_row0 = A.cta_row0.p;
+    rows.doff = A.doff.p;
+    rows.ncta = A.ncta;
+    rows.n = A.N;
+  } else {
+    rows.nb = A.nb;
+  }
+  return rows;
+}
+
+int resident(const void* k, int threads, size_t smem) {
+  int per_sm = 0;
+  BSGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem));
+  return per_sm * num_sms();
+}
+
+void cooperative(const void* kernel, int grid, int threads, size_t smem, void** args, cudaStream_t st) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeCooperative;
+  at.val.cooperative = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  BSGPU_CUDA(cudaLaunchKernelExC(&cfg, kernel, args));
+  BSGPU_CHECK_LAUNCH();
+}
+
+template <typename T, typename ST>
+void run_impl(PcgLaunch& l, const ST* vals, const PcgCall<T>& c, cudaStream_t st) {
+  const Matrix& A = *l.A;
+  PcgCall<T> call = c;
+  double* partial = l.partial.p;
+  uint64_t* packets = l.packets.p;
+  unsigned int* bar = l.bar.p;
+  bool done = false;
+  if (l.kind == PcgLaunch::kSmall) {
+    done = pick_small<T, ST>(A, l.split, [&](auto tag) {
+      using Rows = typename decltype(tag)::Rows;
+      Rows rows = rows_of<Rows>(A, vals);
+      void* args[4] = {&rows, &call, &packets, &bar};
+      cooperative(reinterpret_cast<const void*>(&pcg_small_kernel<Rows>), l.grid, Rows::kT, 0, args, st);
+      return true;
+    });
+  } else {
+    done = pick_large<T, ST>(A, [&](auto tag) {
+      using Rows = typename decltype(tag)::Rows;
+      Rows rows = rows_of<Rows>(A, vals);
+      T* r2 = reinterpret_cast<T*>(l.r2.p);
+      void* args[5] = {&rows, &call, &r2, &partial, &bar};
+      cooperative(reinterpret_cast<const void*>(&pcg_kernel<Rows>), l.grid, Rows::kT, 0, args, st);
+      return true;
+    });
+  }
+  require(done, "CG: no kernel for this matrix", BSGPU_ERR_UNSUPPORTED);
+}
+
+// The small kernel with the widest split of the rows that still gives every CTA one tile, on at most one CTA per SM.
+template <typename T, typename ST>
+bool init_small(PcgLaunch& l) {
+  const Matrix& A = *l.A;
+  for (int w : {4, 2, 1}) {
+    const bool ok = pick_small<T, ST>(A, w, [&](auto tag) {
+      using Rows = typename decltype(tag)::Rows;
+      int64_t tiles = A.ncta;
+      if constexpr (!IsGeneral<Rows>::value) tiles = (A.nb + Rows::BPC - 1) / Rows::BPC;
+      if (tiles > resident(reinterpret_cast<const void*>(&pcg_small_kernel<Rows>), Rows::kT, 0)) return false;
+      l.grid = (int)tiles;
+      return true;
+    });
+    if (!ok) continue;
+    l.kind = PcgLaunch::kSmall;
+    l.split = w;
+    l.packets.alloc(6 * (size_t)l.grid + (size_t)A.N * sizeof(T) / 4);
+    BSGPU_CUDA(cudaMemset(l.packets.p, 0, l.packets.bytes()));
+    return true;
+  }
+  return false;
+}
+
+// The large kernel, up to the sizes at which the separate launches' products (full occupancy) weigh more than what the
+// one launch saves: 24^3 p = 3 FP64 (299 MB) 74 us per iteration against 78, 31^3 (649 MB) 177 against 160; with
+// blocks of 10, 64^3 p = 2 (1.45 GB) 369 against 367.
+template <typename T, typename ST>
+bool init_large(PcgLaunch& l) {
+  const Matrix& A = *l.A;
+  const size_t most = A.uniform && A.Np > 15 ? (size_t)320 << 20 : (size_t)1 << 30;
+  if (A.value_bytes() > most) return false;
+  const bool ok = pick_large<T, ST>(A, [&](auto tag) {
+    using Rows = typename decltype(tag)::Rows;
+    int64_t tiles = A.ncta;
+    if constexpr (!IsGeneral<Rows>::value) tiles = (A.nb + Rows::BPC - 1) / Rows::BPC;
+    l.grid = (int)std::min<int64_t>(tiles, resident(reinterpret_cast<const void*>(&pcg_kernel<Rows>), Rows::kT, 0));
+    return l.grid >= 1;
+  });
+  if (!ok) return false;
+  l.kind = PcgLaunch::kLarge;
+  l.partial.alloc(2 * (size_t)l.grid);
+  l.r2.alloc((size_t)A.N * sizeof(T));
+  return true;
+}
+
+template <typename T, typename ST>
+bool init_impl(PcgLaunch& l) {
+  if (!init_small<T, ST>(l) && !init_large<T, ST>(l)) return false;
+  l.bar.alloc(3);
+  BSGPU_CUDA(cudaMemset(l.bar.p, 0, 3 * sizeof(unsigned int)));
+  return true;
+}
+
+}  // namespace
+
+template <typename T>
+bool PcgLaunch::init(const Matrix& A_) {
+  A = &A_;
+  if (A->N == 0) return false;
+  if constexpr (sizeof(T) == 4) {
+    if (A->half) return init_impl<float, __half>(*this);
+  }
+  return init_impl<T, T>(*this);
+}
+template bool PcgLaunch::init<double>(const Matrix&);
+template bool PcgLaunch::init<float>(const Matrix&);
+
+void pcg_run(PcgLaunch& l, const PcgCall<double>& c, cudaStream_t st) {
+  require(!l.A->single, "precision mismatch");
+  run_impl<double, double>(l, l.A->v64.p, c, st);
+}
+void pcg_run(PcgLaunch& l, const PcgCall<float>& c, cudaStream_t st) {
+  require(l.A->single, "precision mismatch");
+  if (l.A->half) return run_impl<float, __half>(l, l.A->v16.p, c, st);
+  run_impl<float, float>(l, l.A->v32.p, c, st);
+}
+
+}  // namespace bsgpu

@@ -1,0 +1,61 @@
+// Block-preconditioned conjugate gradients (SoftPCG.cs:113-194) as one persistent kernel.
+//
+// All iterations of a solve run inside one cooperative launch.  The CTAs keep their block rows for the whole solve and
+// every CTA adds the per-CTA partial sums in the same fixed order, so all of them take the same decisions and a result
+// does not depend on CTA scheduling.  Small systems (one tile of block rows per CTA) hold the vectors in registers and
+// exchange the direction and the sums as self-validating packets; large ones keep the vectors in memory and meet at
+// counting grid barriers, three per iteration.  Every wait is bounded: one that runs out sets an error word, the other
+// CTAs see it, and the kernel ends.
+#pragma once
+#include "matrix.cuh"
+
+namespace bsgpu {
+
+// Scalars of a solve, in device memory: [0] r.z, [1] p.q, [2] r.z (new), [3] r.r, [4] r0.r0, [5] iterations,
+// [6] beta, [7] state.
+constexpr int kPcgScalars = 8;
+constexpr double kPcgDone = 0.0, kPcgRunning = 1.0, kPcgFailed = 2.0;
+// history entries are written every so many iterations and at the end
+constexpr int kPcgHistory = 8;
+
+// A matrix's CG launch: the kernel, its grid and the scratch of its exchanges, chosen once.
+struct PcgLaunch {
+  enum Kind { kSmall, kLarge };
+  const Matrix* A = nullptr;
+  Kind kind = kLarge;
+  int grid = 0;
+  int split = 1;              // kSmall: threads per DOF row
+  DBuf<unsigned char> r2;     // kLarge: the second residual buffer
+  DBuf<double> partial;       // kLarge: sums per CTA [2 * grid]
+  DBuf<uint64_t> packets;     // kSmall: p.q [2 * grid], r.z and r.r [4 * grid], the direction [N or 2 N]
+  DBuf<unsigned int> bar;     // arrivals (or the epoch of the packets), failure, exits
+  // false: the matrix is served by separate launches (too large, or no kernel for its layout)
+  template <typename T>
+  bool init(const Matrix& A_);
+};
+
+// One call of the solver: x <- solution of A x = b (x: initial guess, known to be zero with `zero`), z = Dinv r with
+// `dinv` (column-major inverse diagonal blocks; null: z = r).  `start` begins a solve, otherwise the launch continues
+// the one in (x, r, z, p, s), a no-op unless s[7] is kPcgRunning; at most `cap` iterations per launch.
+// hist (may be null): sqrt(r.r) at every kPcgHistory-th iteration and at the last one, from entry hist_base on.
+// stop_nonfinite: a NaN/Inf initial residual ends the solve before the first iteration.
+// err (may be null): gets `err_bit` or'ed in when a barrier's wait ran out.
+template <typename T>
+struct PcgCall {
+  T *x, *r, *z, *p, *q;
+  const T* b;
+  const T* dinv;
+  double* s;
+  double* hist;
+  int hist_base, hist_cap;
+  int* err;
+  int err_bit;
+  int mode, max_iter, min_iter;
+  double tol;
+  int zero, start, stop_nonfinite;
+  int cap;
+};
+void pcg_run(PcgLaunch& l, const PcgCall<double>& c, cudaStream_t st);
+void pcg_run(PcgLaunch& l, const PcgCall<float>& c, cudaStream_t st);
+
+}  // namespace bsgpu

@@ -194,6 +194,7 @@ void Ctx::check_graph_errors() {
   *h_err = 0;
   BSGPU_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), st));
   BSGPU_CUDA(cudaStreamSynchronize(st));
+  if (e & kDevErrWait) throw Error(BSGPU_ERR_CUDA, "a kernel's wait for other CTAs ran out");
   if (e & kDevErrSlots) throw Error(BSGPU_ERR_ARITHMETIC, "Orthonormalization: history slots exhausted");
   if (e & kDevErrKrylovNaN) throw Error(BSGPU_ERR_ARITHMETIC, "FlexGMRES: residual is NaN/Inf");
   if (e & kDevErrResidualIncrease) throw Error(BSGPU_ERR_ARITHMETIC, "Orthonormalization: residual increase");
@@ -585,11 +586,12 @@ struct BlockSchwarzT : Solver<T> {
 };
 
 // ---------------------------------------------------------------------------------------------------------------
-// PCG with a block-diagonal preconditioner (SoftPCG.cs:113-194; also the coarsest-level solve).  The iteration
-// runs on device scalars; its kernels are predicated on a device flag that the convergence test clears, so the
-// host launches batches of iterations and reads the state once per batch (the iterate equals that of a test
-// after every iteration).
-// scalars: s[0] rz, s[1] pq, s[2] rz_new, s[3] rr, s[4] rr0, s[5] iterations, s[6] beta, s[7] alpha
+// PCG with a block-diagonal preconditioner (SoftPCG.cs:113-194; also the coarsest-level solve).  Up to the sizes given
+// at PcgLaunch::init the iteration is one persistent kernel (pcg.cuh); driven from the host it runs in launches of at
+// most kCap iterations, after each of which the host reads the scalars and the residual history.  Larger systems run
+// four launches per iteration (nine with blocks that the fused update does not cover) on device scalars, predicated on
+// a device flag that the convergence test clears, so the host launches batches of iterations and reads the state once
+// per batch (the iterate equals that of a test after every iteration).
 // ---------------------------------------------------------------------------------------------------------------
 __global__ void pcg_alpha_kernel(double* s, const int* active) {
   if (*active == 0) return;
@@ -619,27 +621,29 @@ __global__ void pcg_init_kernel(double* s, int* active) {
 
 template <typename T>
 struct PCGT : Solver<T> {
+  static constexpr int kCap = 1024;                 // iterations per launch of the host-driven form
+  static constexpr int kHist = kCap / kPcgHistory;  // history entries of one launch
   const Matrix* A;
   DBuf<T> dinv;
   DBuf<T> r, z, p, q;
-  double* s;
-  int* active;
+  PcgLaunch launch;
+  bool persistent;
+  double* s;  // scalars (pcg.cuh), then the history entries of one launch
   Term term;
-  int batch = 8;
   bool precond;
-  bool use_graph = true;
+  // the form with separate launches
+  static constexpr int batch = kPcgHistory;
+  int* active = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
   const T* graph_X = nullptr;
   long graph_kernels = 0;  // kernels per captured batch (counted at capture time)
   ~PCGT() override {
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
   }
-  void launches_in_graph(Ctx&) { add_launches(graph_kernels); }  // kernels of one replayed batch
   PCGT(Ctx& c, const Matrix* A64, const Matrix* AT, bool use_pc, Term t) : A(AT), term(t), precond(use_pc) {
     const int64_t N = std::max<int64_t>(A->N, 1);
     r.alloc(N); z.alloc(N); p.alloc(N); q.alloc(N);
-    s = c.scal(8);
-    active = c.flag();
+    s = c.scal(kPcgScalars + kHist);
     if (precond) {
       std::vector<int64_t> o = diag_offsets(*A64);
       dinv.alloc(std::max<int64_t>(o.back(), 1));
@@ -650,16 +654,82 @@ struct PCGT : Solver<T> {
         invert_diag_blocks(*A64, nullptr, dinv.p, err, c.st);
       c.check_flag(err, "PCG: singular diagonal block");
     }
-    c.tune(*A, 0);
+    persistent = launch.init<T>(*A);
+    if (!persistent) {
+      active = c.flag();
+      c.tune(*A, 0);
+    }
   }
+  PcgCall<T> call(T* X, const T* B, bool zero) {
+    PcgCall<T> k{};
+    k.x = X;
+    k.b = B;
+    k.r = r.p;
+    k.z = z.p;
+    k.p = p.p;
+    k.q = q.p;
+    k.dinv = precond ? dinv.p : nullptr;
+    k.s = s;
+    k.mode = term.mode;
+    k.tol = term.tol;
+    k.max_iter = term.max_iter;
+    k.min_iter = term.min_iter;
+    k.zero = zero ? 1 : 0;
+    k.start = 1;
+    return k;
+  }
+  void solve(Ctx& c, T* X, const T* B, bool zero) override {
+    TraceScope ts(c, this->trace);
+    if (!persistent) return solve_launches(c, X, B, zero);
+    PcgCall<T> k = call(X, B, zero);
+    k.stop_nonfinite = 1;
+    k.cap = kCap;
+    k.hist = s + kPcgScalars;
+    k.hist_cap = kHist;
+    const double* hs = c.hscal + (s - c.dscal.p);
+    double R0 = 0, R = 0;
+    int it = 0;
+    while (true) {
+      pcg_run(launch, k, c.st);
+      c.fetch(s, kPcgScalars + kHist);
+      if (hs[7] == kPcgFailed) throw Error(BSGPU_ERR_CUDA, "PCG: a wait for other CTAs ran out");
+      if (k.start) {
+        R0 = std::sqrt(hs[4]);
+        this->history.assign(1, R0);
+        if (!std::isfinite(R0)) throw Error(BSGPU_ERR_ARITHMETIC, "PCG: NaN/Inf in the initial residual");
+      }
+      it = (int)hs[5];
+      for (int e = 0; (k.hist_base + e) * kPcgHistory < it; ++e) this->history.push_back(hs[kPcgScalars + e]);
+      R = std::sqrt(hs[3]);
+      if (!std::isfinite(hs[3]) || !std::isfinite(hs[2])) throw Error(BSGPU_ERR_ARITHMETIC, "PCG: NaN/Inf");
+      if (hs[7] == kPcgDone) break;
+      k.start = 0;
+      k.hist_base = it / kPcgHistory;
+    }
+    this->converged = term(it, R0, R).second;
+    this->this_level_iterations = it;
+    if (c.tracing && this->trace >= 0) c.trace[this->trace].iterations += it;
+  }
+  bool graphable() const override { return term.max_iter <= kMaxRecordedIterations && term.min_iter <= term.max_iter; }
+  // recorded form: the whole solve is the one launch; it ends at the latest when the iteration count passes max_iter
+  void solve_graph(Ctx& c, T* X, const T* B, bool zero) override {
+    require(graphable(), "coarse CG: iteration limits cannot be recorded");
+    if (!persistent) return record_launches(c, X, B, zero);
+    PcgCall<T> k = call(X, B, zero);
+    k.cap = kMaxRecordedIterations + 1;
+    k.err = c.d_err;
+    k.err_bit = kDevErrWait;
+    pcg_run(launch, k, c.st);
+  }
+
+  // ---- separate launches ----
   void apply_pc(Ctx& c, const T* in, T* out, const int* act) {
     if (precond)
       blockdiag_apply(*A, dinv.p, T(1), in, out, c.st, act);
     else
       copy_vec(out, in, A->N, c.st);
   }
-  void solve(Ctx& c, T* X, const T* B, bool zero) override {
-    TraceScope ts(c, this->trace);
+  void solve_launches(Ctx& c, T* X, const T* B, bool zero) {
     const int64_t N = A->N;
     cudaStream_t st = c.st;
     if (zero)
@@ -684,48 +754,16 @@ struct PCGT : Solver<T> {
     double R = R0;
     if (!std::isfinite(R0)) throw Error(BSGPU_ERR_ARITHMETIC, "PCG: NaN/Inf in the initial residual");
     if (st0.first) {
-      const int grid = elt_grid(N);
-      const bool fused = precond && A->uniform && A->nb > 0 &&
-                         (A->Np == 4 || A->Np == 6 || A->Np == 10 || A->Np == 20);
-      const T* px[1] = {p.p};
-      const T* qx[1] = {q.p};
-      auto batch_kernels = [&]() {
-        for (int bi = 0; bi < batch; ++bi) {
-          spmv(*A, T(1), p.p, T(0), (const T*)nullptr, q.p, st, active);
-          dots(c.red, 1, px, qx, N, s + 1, 0, st, active);
-          if (fused) {
-            // alpha, x and r updates, z = Dinv r, r.z, r.r and the beta / termination step in one launch
-            pcg_update(c.red, A->Np, s, active, X, p.p, q.p, r.p, z.p, dinv.p, A->nb, term.mode, term.tol,
-                       term.max_iter, term.min_iter, st);
-            xpby_kernel<T><<<grid, 256, 0, st>>>(z.p, s + 6, p.p, N, active);
-            BSGPU_CHECK_LAUNCH();
-            continue;
-          }
-          pcg_alpha_kernel<<<1, 1, 0, st>>>(s, active);
-          BSGPU_CHECK_LAUNCH();
-          axpys(1, s + 7, nullptr, 1.0, px, X, N, st, active);
-          axpys(1, s + 7, nullptr, -1.0, qx, r.p, N, st, active);
-          apply_pc(c, r.p, z.p, active);
-          {
-            const T* a[2] = {r.p, r.p};
-            const T* b[2] = {z.p, r.p};
-            dots(c.red, 2, a, b, N, s + 2, 0, st, active);
-          }
-          pcg_beta_kernel<<<1, 1, 0, st>>>(s, active, term.mode, term.tol, term.max_iter, term.min_iter);
-          xpby_kernel<T><<<grid, 256, 0, st>>>(z.p, s + 6, p.p, N, active);
-          BSGPU_CHECK_LAUNCH();
-        }
-      };
       // the batch is captured once per solution vector and replayed as one CUDA graph launch (its kernels,
       // predicated on `active`, become no-ops once converged)
-      if (use_graph && (graph_exec == nullptr || graph_X != X)) {
+      if (graph_exec == nullptr || graph_X != X) {
         if (graph_exec) cudaGraphExecDestroy(graph_exec);
         graph_exec = nullptr;
         cudaGraph_t g = nullptr;
         BSGPU_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         try {
           const unsigned long long n0 = launches_now();
-          batch_kernels();
+          for (int bi = 0; bi < batch; ++bi) iteration_kernels(c, X);
           graph_kernels = (long)(launches_now() - n0);
           add_launches(-(long long)graph_kernels);
         } catch (...) {
@@ -739,12 +777,8 @@ struct PCGT : Solver<T> {
         graph_X = X;
       }
       while (true) {
-        if (use_graph) {
-          BSGPU_CUDA(cudaGraphLaunch(graph_exec, st));
-          launches_in_graph(c);
-        } else {
-          batch_kernels();
-        }
+        BSGPU_CUDA(cudaGraphLaunch(graph_exec, st));
+        add_launches(graph_kernels);
         int h_active = 0;
         BSGPU_CUDA(cudaMemcpyAsync(&h_active, active, sizeof(int), cudaMemcpyDeviceToHost, st));
         c.fetch(s, 8);
@@ -762,11 +796,9 @@ struct PCGT : Solver<T> {
     this->this_level_iterations = it;
     if (c.tracing && this->trace >= 0) c.trace[this->trace].iterations += it;
   }
-  bool graphable() const override { return term.max_iter <= kMaxRecordedIterations && term.min_iter <= term.max_iter; }
   // Recorded form: the initialisation, then a WHILE node whose body is one CG iteration; the fused update's
   // termination step clears `active` (at the latest when the iteration count passes max_iter), which ends the loop.
-  void solve_graph(Ctx& c, T* X, const T* B, bool zero) override {
-    require(graphable(), "coarse CG: iteration limits cannot be recorded");
+  void record_launches(Ctx& c, T* X, const T* B, bool zero) {
     const int64_t N = A->N;
     if (zero)
       copy_vec(r.p, B, N, c.st);

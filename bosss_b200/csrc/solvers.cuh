@@ -14,6 +14,7 @@
 #include "devctl.cuh"
 #include "learned.cuh"
 #include "matrix.cuh"
+#include "pcg.cuh"
 
 namespace bsgpu {
 
