@@ -200,6 +200,7 @@ void solve_device(bsgpu_solver_s* s, double* dX, const double* dB, bsgpu_solve_s
   BSGPU_CUDA(cudaEventRecord(s->e1, c.st));
   BSGPU_CUDA(cudaEventSynchronize(s->e1));
   c.flush_graph_counts();
+  c.check_graph_errors();
   if (t.net) learned_check(*t.net, c.st);
   float ms = 0;
   BSGPU_CUDA(cudaEventElapsedTime(&ms, s->e0, s->e1));

@@ -1,0 +1,239 @@
+// Natural-order block ILU(0) application (see ilu.cuh).
+#include <algorithm>
+
+#include "ilu.cuh"
+#include "ldst.cuh"
+#include "packets.cuh"
+
+namespace bsgpu {
+
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kWarps = kThreads / 32;
+
+// One warp per block row; the warps take the rows in wavefront order (warp w the rows w, w + W, ...), first those of
+// the forward pass y_i = b_i - sum_{k<i} L_ik y_k, then those of x_i = U_ii^{-1} (y_i - sum_{j>i} U_ij x_j).
+// A row waits for exactly the rows it needs: their values arrive as packets.  All CTAs are resident (cooperative
+// launch) and a row only needs rows before it in its pass, so the first unfinished row can always proceed.
+// 32 / NP lanes share a DOF row (one neighbour block each); the operand block is fetched one value per lane and
+// handed round by shuffles.
+// Bound by the chain of wavefronts: each costs one store-to-load handover through L2 (1.0 to 1.7 us) instead of a
+// launch (14 us), and the passes read the lower and the upper blocks once each instead of whole rows twice.  28^3 p = 2
+// FP64 (119 MB, 164 wavefronts): 2.3 ms as one launch per wavefront and pass, 0.20 ms now; 48^3 p = 2 (608 MB) 0.38 ms.
+template <typename T, int NP, int V>
+__global__ void __launch_bounds__(kThreads) ilu_apply_kernel(
+    const int64_t* __restrict__ rp, const int32_t* __restrict__ ci, const int64_t* __restrict__ diag,
+    const int32_t* __restrict__ order, const int32_t* __restrict__ rorder, const T* __restrict__ vals, const T* __restrict__ uinv,
+    const T* __restrict__ b, T* __restrict__ x, int64_t nb, uint64_t* __restrict__ packets,
+    unsigned int* __restrict__ state, int* __restrict__ err, int err_bit) {
+  constexpr int SPLIT = 32 / NP;
+  constexpr int WPV = sizeof(T) / 4;
+  constexpr unsigned ALL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int s = lane / NP, r = lane - s * NP;
+  const bool lane_used = s < SPLIT;
+  const int64_t W = (int64_t)gridDim.x * kWarps;
+  const int64_t w0 = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;  // neighbouring rows on different SMs
+  const unsigned ep = state[0] + 1u;
+  unsigned int* const fail = state + 1;
+  uint64_t* const yp = packets;
+  uint64_t* const xp = packets + nb * NP * WPV;
+  const uint64_t pol = policy_evict_first();
+
+  // Sum over the blocks [k0, k1) of block * operand, in the lanes s = 0.  The blocks of ROUNDS rounds (SPLIT blocks
+  // each) are loaded before the first wait, so that on a Cartesian grid only the operand is waited for; `op` holds the
+  // packets of all rows, or with `scale` 0 one row's packets for every block.
+  constexpr int ROUNDS = SPLIT >= 3 ? 1 : 3 / SPLIT;
+  auto product = [&](int64_t k0, int64_t k1, const uint64_t* op, int scale) {
+    T acc[2] = {0, 0};
+    for (int64_t kk = k0; kk < k1; kk += SPLIT * ROUNDS) {
+      T a[ROUNDS][NP];
+      const uint64_t* w[ROUNDS];
+      T xv[ROUNDS];
+#pragma unroll
+      for (int h = 0; h < ROUNDS; ++h) {
+        const int64_t k = kk + h * SPLIT + s;
+        w[h] = nullptr;
+        xv[h] = 0;
+        if (lane_used && k < k1) {
+          w[h] = op + ((int64_t)__ldg(ci + k) * NP * scale + r) * WPV;
+          const T* vb = vals + k * (NP * NP) + r * V;
+#pragma unroll
+          for (int c = 0; c < NP / V; ++c) {
+            const Vec<T, V> v = ldv_stream<T, V>(vb + c * (NP * V), pol);
+#pragma unroll
+            for (int q = 0; q < V; ++q) a[h][c * V + q] = v.a[q];
+          }
+        }
+      }
+      warp_wait(fail, [&] {
+        bool ready = true;
+#pragma unroll
+        for (int h = 0; h < ROUNDS; ++h)
+          if (w[h] != nullptr) ready = load_packet(w[h], ep, xv[h]) && ready;
+        return ready;
+      });
+#pragma unroll
+      for (int h = 0; h < ROUNDS; ++h) {
+#pragma unroll
+        for (int c = 0; c < NP; ++c) {
+          const T xc = __shfl_sync(ALL, xv[h], lane_used ? s * NP + c : 0);
+          if (w[h] != nullptr) acc[c & 1] = fma(a[h][c], xc, acc[c & 1]);
+        }
+      }
+    }
+    const T mine = acc[0] + acc[1];
+    T sum = mine;
+#pragma unroll
+    for (int q = 1; q < SPLIT; ++q) sum += __shfl_sync(ALL, mine, r + q * NP < 32 ? r + q * NP : 0);
+    return sum;
+  };
+
+  // Each pass begins with one row (n < 0) whose operand is a packet of the warp's own and whose result goes nowhere:
+  // it brings the pass's instructions into the SM's cache while nobody waits for it (an instruction miss on the chain
+  // of wavefronts costs more than a wavefront).
+  uint64_t* const own = packets + (2 * nb + w0) * NP * WPV;
+  if (s == 0) put_packet(own + r * WPV, T(0), ep);
+  for (int64_t n = w0 - W; n < nb; n += W) {
+    const bool real = n >= 0;
+    const int64_t i = __ldg(order + (real ? n : nb - 1));
+    const int64_t g = i * NP + r;
+    const T bi = s == 0 ? b[g] : T(0);
+    const T sum = product(__ldg(rp + i), __ldg(diag + i), real ? yp : own, real ? 1 : 0);
+    if (s == 0) put_packet(real ? yp + g * WPV : own + r * WPV, bi - sum, ep);
+  }
+  for (int64_t n = w0 - W; n < nb; n += W) {
+    const bool real = n >= 0;
+    const int64_t i = __ldg(rorder + (real ? n : nb - 1));
+    const int64_t g = i * NP + r;
+    // the inverse's columns s, s + SPLIT, ... of this lane's row
+    constexpr int NC = (NP + SPLIT - 1) / SPLIT;
+    T d[NC];
+    const T* D = uinv + i * (NP * NP) + r;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) d[c] = (lane_used && c * SPLIT + s < NP) ? __ldg(D + (c * SPLIT + s) * NP) : T(0);
+    T yi = 0;
+    const uint64_t* const yw = real ? yp + g * WPV : own + r * WPV;
+    warp_wait(fail, [&] { return s != 0 || load_packet(yw, ep, yi); });
+    const T sum = product(__ldg(diag + i) + 1, __ldg(rp + i + 1), real ? xp : own, real ? 1 : 0);
+    const T q = yi - sum;
+    T z = 0;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int col = c * SPLIT + s;
+      const T qc = __shfl_sync(ALL, q, col < NP ? col : 0);
+      z = fma(d[c], qc, z);
+    }
+    T tot = z;
+#pragma unroll
+    for (int p = 1; p < SPLIT; ++p) tot += __shfl_sync(ALL, z, r + p * NP < 32 ? r + p * NP : 0);
+    if (s == 0) {
+      put_packet(real ? xp + g * WPV : own + r * WPV, tot, ep);
+      if (real) x[g] = tot;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(state + 2, 1u) == gridDim.x - 1) {
+      if (*(volatile unsigned int*)fail) atomicOr(err, err_bit);
+      state[0] = ep;
+      state[1] = state[2] = 0u;
+    }
+  }
+}
+
+template <typename T, typename F>
+void with_kernel(const Matrix& M, F&& f) {
+#define BSGPU_ILU(NP, VV) \
+  if (M.Np == NP && M.V == VV) return f(&ilu_apply_kernel<T, NP, VV>);
+  if constexpr (sizeof(T) == 8) {
+    BSGPU_ILU(4, 2) BSGPU_ILU(20, 2)
+  } else {
+    BSGPU_ILU(4, 4) BSGPU_ILU(20, 4)
+  }
+  BSGPU_ILU(6, 2) BSGPU_ILU(10, 2)
+#undef BSGPU_ILU
+  throw Error(BSGPU_ERR_UNSUPPORTED, "natural-order ILU needs uniform blocks of 4, 6, 10 or 20");
+}
+
+template <typename T>
+void apply_impl(IluApply& a, const T* vals, const T* uinv, const T* b, T* x, int* err, int err_bit, cudaStream_t st) {
+  const Matrix& M = *a.M;
+  if (M.nb == 0) return;
+  with_kernel<T>(M, [&](auto* kernel) {
+    const int64_t* rp = M.rp.p;
+    const int32_t* ci = M.ci.p;
+    const int64_t* diag = a.diag.p;
+    const int32_t* order = a.order.p;
+    const int32_t* rorder = a.rorder.p;
+    int64_t nb = M.nb;
+    uint64_t* packets = a.packets.p;
+    unsigned int* state = a.state.p;
+    void* args[] = {&rp, &ci, &diag, &order, &rorder, &vals, &uinv, &b, &x, &nb, &packets, &state, &err, &err_bit};
+    BSGPU_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3((unsigned)a.grid),
+                                           dim3(kThreads), args, 0, st));
+    BSGPU_CHECK_LAUNCH();
+  });
+}
+
+}  // namespace
+
+void IluApply::init(const Matrix& M_, const std::vector<int64_t>& lptr, const std::vector<int32_t>& order_) {
+  M = &M_;
+  const int64_t nb = M->nb;
+  if (nb == 0) return;
+  require(M->uniform && !M->half, "natural-order ILU needs uniform blocks of FP64 or FP32 values");
+  std::vector<int64_t> d(nb, -1);
+  for (int64_t i = 0; i < nb; ++i)
+    for (int64_t k = M->h_rp[i]; k < M->h_rp[i + 1]; ++k)
+      if (M->h_ci[k] == i) d[i] = k;
+  for (int64_t i = 0; i < nb; ++i) require(d[i] >= 0, "ILU: a diagonal block is missing", BSGPU_ERR_ARITHMETIC);
+  // backward wavefronts: one more than the largest of the upper neighbours
+  std::vector<int32_t> lev(nb, 0), back(nb);
+  int nlev = 0;
+  for (int64_t i = nb - 1; i >= 0; --i) {
+    for (int64_t k = d[i] + 1; k < M->h_rp[i + 1]; ++k) lev[i] = std::max(lev[i], lev[M->h_ci[k]] + 1);
+    nlev = std::max(nlev, lev[i] + 1);
+  }
+  std::vector<int64_t> at(nlev + 1, 0);
+  for (int64_t i = 0; i < nb; ++i) at[lev[i] + 1]++;
+  for (int l = 0; l < nlev; ++l) at[l + 1] += at[l];
+  for (int64_t i = 0; i < nb; ++i) back[at[lev[i]]++] = (int32_t)i;
+  order.alloc(nb);
+  rorder.alloc(nb);
+  BSGPU_CUDA(cudaMemcpy(rorder.p, back.data(), nb * 4, cudaMemcpyHostToDevice));
+  diag.alloc(nb);
+  BSGPU_CUDA(cudaMemcpy(order.p, order_.data(), nb * 4, cudaMemcpyHostToDevice));
+  BSGPU_CUDA(cudaMemcpy(diag.p, d.data(), nb * 8, cudaMemcpyHostToDevice));
+  const size_t words = M->single ? 1 : 2;
+  state.alloc(3);
+  BSGPU_CUDA(cudaMemset(state.p, 0, 3 * sizeof(unsigned int)));
+  // warps for two of the widest wavefronts: while one is being computed the blocks of the next are on their way
+  int64_t widest = 1;
+  for (size_t l = 0; l + 1 < lptr.size(); ++l) widest = std::max(widest, lptr[l + 1] - lptr[l]);
+  int per_sm = 0;
+  auto occ = [&](auto* kernel) {
+    BSGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, 0));
+  };
+  if (M->single)
+    with_kernel<float>(*M, occ);
+  else
+    with_kernel<double>(*M, occ);
+  require(per_sm >= 1, "ILU: the kernel does not fit the device", BSGPU_ERR_UNSUPPORTED);
+  grid = (int)std::min<int64_t>((2 * widest + kWarps - 1) / kWarps, (int64_t)per_sm * num_sms());
+  packets.alloc((2 * (size_t)M->N + (size_t)grid * kWarps * M->Np) * words);
+  BSGPU_CUDA(cudaMemset(packets.p, 0, packets.bytes()));
+}
+
+void ilu_apply(IluApply& a, const double* uinv, const double* b, double* x, int* err, int err_bit, cudaStream_t st) {
+  require(!a.M->single, "precision mismatch");
+  apply_impl<double>(a, a.M->v64.p, uinv, b, x, err, err_bit, st);
+}
+void ilu_apply(IluApply& a, const float* uinv, const float* b, float* x, int* err, int err_bit, cudaStream_t st) {
+  require(a.M->single, "precision mismatch");
+  apply_impl<float>(a, a.M->v32.p, uinv, b, x, err, err_bit, st);
+}
+
+}  // namespace bsgpu

@@ -1,0 +1,23 @@
+// Application of a block ILU(0) in the natural block-row order (CellILU.Solve, CellILU.cs:182-250) as one launch.
+#pragma once
+#include "matrix.cuh"
+
+namespace bsgpu {
+
+struct IluApply {
+  const Matrix* M = nullptr;      // unit-lower L below the diagonal, U on and above it (uniform blocks of 4, 6, 10, 20)
+  DBuf<int32_t> order, rorder;    // block rows, wavefront by wavefront, for the forward and the backward pass
+  DBuf<int64_t> diag;             // index of every block row's diagonal block
+  DBuf<uint64_t> packets;         // y and x of every row, and one row per warp
+  DBuf<unsigned int> state;       // epoch, failure, exits
+  int grid = 0;
+  // lptr: offsets of the wavefronts in `order`
+  void init(const Matrix& M_, const std::vector<int64_t>& lptr, const std::vector<int32_t>& order_);
+};
+
+// x = U^{-1} L^{-1} b; uinv: inverses of U's diagonal blocks, column-major at diag_offsets(M).  err gets `err_bit`
+// or'ed in when a row's wait for its neighbours ran out.
+void ilu_apply(IluApply& a, const double* uinv, const double* b, double* x, int* err, int err_bit, cudaStream_t st);
+void ilu_apply(IluApply& a, const float* uinv, const float* b, float* x, int* err, int err_bit, cudaStream_t st);
+
+}  // namespace bsgpu

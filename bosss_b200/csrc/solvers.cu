@@ -201,6 +201,12 @@ void Ctx::check_graph_errors() {
   throw Error(BSGPU_ERR_ARITHMETIC, "Orthonormalization: NaN/Inf in the preconditioner");
 }
 
+void Ctx::queue_error() {
+  if (capturing) return;  // read after the graph
+  BSGPU_CUDA(cudaMemcpyAsync(h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  err_pending = true;
+}
+
 void Ctx::flush_graph_counts() {
   if (!graph_ran) return;
   graph_ran = false;
@@ -451,12 +457,9 @@ struct ILU0T : Solver<T> {
 // Block ILU(0) smoother in the reference's natural cell order (CellILU.cs:22; ComputeILU :1229-1330, Solve
 // :182-250).  The dependency chain of the natural order is cut into wavefronts (block rows whose lower neighbours
 // all lie in earlier wavefronts; 3n-2 of them on an n^3 Cartesian grid): the factorisation is one launch per
-// wavefront (ilu0_levels), and x = U^{-1} L^{-1} b is one launch per wavefront and pass: the forward pass
-// y_i = b_i - sum_{k<i} L_ik y_k over the wavefronts in order, the backward pass x_i = U_ii^{-1} (y_i - sum_{j>i}
-// U_ij x_j) in reverse order, both as in-place row updates on zero-initialised vectors (rows not yet visited are
-// zero, so the full row product only sees the finished neighbours).  Factors computed in FP64, stored and applied
-// in FP32 for the mixed-precision preconditioner (the reference's single-precision back substitution,
-// CellILU.cs:914).
+// wavefront (ilu0_levels), and x = U^{-1} L^{-1} b one launch for both passes (ilu.cuh), in which a row waits for the
+// values of its neighbours and not for whole wavefronts.  Factors computed in FP64, stored and applied in FP32 for the
+// mixed-precision preconditioner (the reference's single-precision back substitution, CellILU.cs:914).
 template <typename T>
 struct ILUNaturalT : Solver<T> {
   bool graphable() const override { return true; }
@@ -464,16 +467,15 @@ struct ILUNaturalT : Solver<T> {
   const Matrix* M = nullptr;
   DBuf<double> uinv64;
   DBuf<float> uinv32;
-  DBuf<int32_t> rows;
-  std::vector<int64_t> lptr;
-  DBuf<T> y;
+  IluApply apply;
   ILUNaturalT(Ctx& c, const Matrix* A64) {
     require(A64->uniform && (A64->Np == 4 || A64->Np == 6 || A64->Np == 10 || A64->Np == 20),
             "natural-order ILU needs uniform blocks of 4, 6, 10 or 20", BSGPU_ERR_UNSUPPORTED);
     const int64_t nb = A64->nb;
     std::vector<int32_t> order;
+    std::vector<int64_t> lptr;
     ilu_wavefronts(*A64, lptr, order);
-    rows.alloc(std::max<int64_t>(nb, 1));
+    DBuf<int32_t> rows(std::max<int64_t>(nb, 1));
     if (nb) BSGPU_CUDA(cudaMemcpy(rows.p, order.data(), nb * 4, cudaMemcpyHostToDevice));
     const std::vector<int64_t> o = diag_offsets(*A64);
     uinv64.alloc(std::max<int64_t>(o.back(), 1));
@@ -491,7 +493,8 @@ struct ILUNaturalT : Solver<T> {
     } else {
       M = M64.get();
     }
-    y.alloc(std::max<int64_t>(M->N, 1));
+    apply.init(*M, lptr, order);
+    c.graph_init();  // the error word
   }
   const T* uinv() const {
     if constexpr (sizeof(T) == 4)
@@ -499,16 +502,11 @@ struct ILUNaturalT : Solver<T> {
     else
       return uinv64.p;
   }
-  int wavefronts() const { return (int)lptr.size() - 1; }
   void solve(Ctx& c, T* X, const T* B, bool zero) override {
     (void)zero;  // CellILU overwrites X
     TraceScope ts(c, this->trace);
-    const int L = wavefronts();
-    fill(T(0), y.p, M->N, c.st);
-    for (int l = 0; l < L; ++l) unit_update_rows(*M, rows.p + lptr[l], lptr[l + 1] - lptr[l], B, y.p, c.st);
-    fill(T(0), X, M->N, c.st);
-    for (int l = L - 1; l >= 0; --l)
-      gs_update_rows(*M, uinv(), T(1), rows.p + lptr[l], lptr[l + 1] - lptr[l], y.p, X, c.st);
+    if (M->nb) ilu_apply(apply, uinv(), B, X, c.d_err, kDevErrWait, c.st);
+    c.queue_error();
     this->this_level_iterations++;
     this->converged = true;
   }

@@ -12,6 +12,7 @@
 #include "blockops.cuh"
 #include "bschwarz.cuh"
 #include "devctl.cuh"
+#include "ilu.cuh"
 #include "learned.cuh"
 #include "matrix.cuh"
 #include "pcg.cuh"
@@ -92,6 +93,7 @@ struct Ctx {
   cudaGraphConditionalHandle cond_handle();
   void cond_begin(cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type, int body);
   void cond_end();
+  void queue_error();         // queues a copy of the error word (outside a recording)
   void check_graph_errors();  // after a synchronisation: raises the pending device error, if any
   void flush_graph_counts();  // synchronises; adds the kernels of the conditional bodies that ran
 };
