@@ -1,5 +1,6 @@
 // Device-side control flow of the graph-captured V-cycle (see devctl.cuh).
 #include <algorithm>
+#include <initializer_list>
 
 #include "devctl.cuh"
 
@@ -94,16 +95,18 @@ __global__ void __launch_bounds__(kThreads) hist_dots_kernel(const T* const* __r
                                                              const T* __restrict__ m, int64_t n,
                                                              double* __restrict__ beta, double* __restrict__ self,
                                                              double* __restrict__ partial,
-                                                             unsigned int* __restrict__ ticket) {
+                                                             unsigned int* __restrict__ ticket,
+                                                             const int* __restrict__ active) {
   using V = typename V16<T>::type;
   constexpr int W = V16<T>::W;
+  if (active != nullptr && *active == 0) return;
   const int k = min(*kp, kmax);
   const int j0 = blockIdx.y * kChunk;
   const int K = max(0, min(kChunk, k - j0));
   const bool do_self = self != nullptr && blockIdx.y == 0;
   if (K == 0 && !do_self) return;
   __shared__ const T* ptr[kChunk];
-  if (threadIdx.x < K) ptr[threadIdx.x] = hist[j0 + threadIdx.x];
+  if (threadIdx.x < kChunk) ptr[threadIdx.x] = threadIdx.x < K ? hist[j0 + threadIdx.x] : nullptr;
   __syncthreads();
   double acc[kProducts];
 #pragma unroll
@@ -113,9 +116,16 @@ __global__ void __launch_bounds__(kThreads) hist_dots_kernel(const T* const* __r
   const V* mv = reinterpret_cast<const V*>(m);
   for (int64_t j = (int64_t)blockIdx.x * kThreads + threadIdx.x; j < nv; j += stride) {
     const V bb = __ldg(mv + j);
+    // eight vectors' pieces in flight before the first is used: 16 vectors of 2.6M FP32 values in 45 us, 81 us with
+    // each product waiting for its own load
 #pragma unroll
-    for (int q = 0; q < kChunk; ++q)
-      if (q < K) acc[q] += vdot(__ldcs(reinterpret_cast<const V*>(ptr[q]) + j), bb);
+    for (int q0 = 0; q0 < kChunk; q0 += 8) {
+      V a[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) a[q] = q0 + q < K ? reinterpret_cast<const V*>(ptr[q0 + q])[j] : V{};
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[q0 + q] += vdot(a[q], bb);
+    }
     if (do_self) acc[kChunk] += vdot(bb, bb);
   }
   for (int64_t i = nv * W + (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += stride) {
@@ -165,16 +175,62 @@ __global__ void __launch_bounds__(kThreads) hist_dots_kernel(const T* const* __r
   if (threadIdx.x == 0) ticket[blockIdx.y] = 0u;
 }
 
+// Last half of a one-value grid sum: true in the CTA that arrives last, with the total (fixed order) in its thread 0.
+__device__ __forceinline__ bool grid_total(double v, double* __restrict__ partial, unsigned int* __restrict__ ticket,
+                                           double* total) {
+  __shared__ double red[kThreads / 32];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  v = warp_sum(v);
+  if (lane == 0) red[warp] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) s += red[w];
+    __stcg(partial + blockIdx.x, s);
+    __threadfence();
+    last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  double s = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += kThreads) s += __ldcg(partial + b);
+  s = warp_sum(s);
+  __syncthreads();
+  if (lane == 0) red[warp] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double tot = 0.0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) tot += red[w];
+    *total = tot;
+    *ticket = 0u;
+  }
+  return true;
+}
+
+// y1 -= sum_{j<k} beta_j x1_j, y2 -= sum_{j<k} beta_j x2_j and |y2| into proj[0]; the last CTA then takes AddSol's
+// decision.  Bound by HBM: 2 k vectors read ((2 k + 4) N values); four history entries in flight per thread, 2.6M FP32
+// unknowns and k = 43: 170 us, 217 with one entry in flight.  sweep 1: the norm of the correction's image before (nM) and after the projection, relative (rel), and
+// whether a second sweep restores orthogonality (1e-5 < rel < 0.5, "twice is enough"; the cancellation bound 1e-5 of
+// OrthonormalizationMultigrid.cs:263-337); with an empty history there is nothing to project and rel = 1.  sweep 2
+// (only where s->second is set): rel after it.
 template <typename T>
-__global__ void __launch_bounds__(kThreads) hist_axpy2_kernel(const T* const* __restrict__ x1,
-                                                              const T* const* __restrict__ x2,
-                                                              const int* __restrict__ kp, int kmax,
-                                                              const double* __restrict__ beta, T* __restrict__ y1,
-                                                              T* __restrict__ y2, int64_t n) {
+__global__ void __launch_bounds__(kThreads) ortho_project_kernel(const T* const* __restrict__ x1,
+                                                                 const T* const* __restrict__ x2,
+                                                                 OrthoState* __restrict__ s, int kmax, int sweep,
+                                                                 const double* __restrict__ beta, T* __restrict__ y1,
+                                                                 T* __restrict__ y2, int64_t n,
+                                                                 double* __restrict__ proj,
+                                                                 double* __restrict__ partial,
+                                                                 unsigned int* __restrict__ ticket,
+                                                                 int* __restrict__ err) {
   using V = typename V16<T>::type;
   constexpr int W = V16<T>::W;
-  const int k = min(*kp, min(kmax, kHistMax));
-  if (k <= 0) return;
+  if (sweep == 2 && s->second == 0) return;
+  const int k = max(0, min(s->k, min(kmax, kHistMax)));
   __shared__ const T* p1[kHistMax];
   __shared__ const T* p2[kHistMax];
   __shared__ double c[kHistMax];
@@ -186,32 +242,49 @@ __global__ void __launch_bounds__(kThreads) hist_axpy2_kernel(const T* const* __
   __syncthreads();
   const int64_t nv = n / W;
   const int64_t stride = (int64_t)gridDim.x * kThreads;
-  for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < nv; i += stride) {
+  double sq = 0.0;
+  // from the end: hist_dots has just read the images there, and L2 still holds them
+  for (int64_t i = nv - 1 - ((int64_t)blockIdx.x * kThreads + threadIdx.x); i >= 0; i -= stride) {
     double a1[W], a2[W];
 #pragma unroll
     for (int w = 0; w < W; ++w) a1[w] = a2[w] = 0.0;
-    for (int j = 0; j < k; ++j) {
-      const V u = __ldcs(reinterpret_cast<const V*>(p1[j]) + i);
-      const V v = __ldcs(reinterpret_cast<const V*>(p2[j]) + i);
-      const T* uu = reinterpret_cast<const T*>(&u);
-      const T* vv = reinterpret_cast<const T*>(&v);
+    // four history entries' pieces in flight before the first is used
+    for (int j0 = 0; j0 < k; j0 += 4) {
+      V u[4], v[4];
+      double cc[4];
 #pragma unroll
-      for (int w = 0; w < W; ++w) {
-        a1[w] = fma(c[j], (double)uu[w], a1[w]);
-        a2[w] = fma(c[j], (double)vv[w], a2[w]);
+      for (int q = 0; q < 4; ++q) {
+        const bool on = j0 + q < k;
+        u[q] = on ? __ldcs(reinterpret_cast<const V*>(p1[j0 + q]) + i) : V{};
+        v[q] = on ? __ldcs(reinterpret_cast<const V*>(p2[j0 + q]) + i) : V{};
+        cc[q] = on ? c[j0 + q] : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const T* uu = reinterpret_cast<const T*>(&u[q]);
+        const T* vv = reinterpret_cast<const T*>(&v[q]);
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          a1[w] = fma(cc[q], (double)uu[w], a1[w]);
+          a2[w] = fma(cc[q], (double)vv[w], a2[w]);
+        }
       }
     }
-    V o1 = reinterpret_cast<V*>(y1)[i];
     V o2 = reinterpret_cast<V*>(y2)[i];
-    T* oo1 = reinterpret_cast<T*>(&o1);
     T* oo2 = reinterpret_cast<T*>(&o2);
+    if (k > 0) {
+      V o1 = reinterpret_cast<V*>(y1)[i];
+      T* oo1 = reinterpret_cast<T*>(&o1);
 #pragma unroll
-    for (int w = 0; w < W; ++w) {
-      oo1[w] = (T)((double)oo1[w] - a1[w]);
-      oo2[w] = (T)((double)oo2[w] - a2[w]);
+      for (int w = 0; w < W; ++w) {
+        oo1[w] = (T)((double)oo1[w] - a1[w]);
+        oo2[w] = (T)((double)oo2[w] - a2[w]);
+      }
+      reinterpret_cast<V*>(y1)[i] = o1;
+      reinterpret_cast<V*>(y2)[i] = o2;
     }
-    reinterpret_cast<V*>(y1)[i] = o1;
-    reinterpret_cast<V*>(y2)[i] = o2;
+#pragma unroll
+    for (int w = 0; w < W; ++w) sq = fma((double)oo2[w], (double)oo2[w], sq);
   }
   for (int64_t i = nv * W + (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += stride) {
     double a1 = 0.0, a2 = 0.0;
@@ -219,17 +292,22 @@ __global__ void __launch_bounds__(kThreads) hist_axpy2_kernel(const T* const* __
       a1 = fma(c[j], (double)p1[j][i], a1);
       a2 = fma(c[j], (double)p2[j][i], a2);
     }
-    y1[i] = (T)((double)y1[i] - a1);
-    y2[i] = (T)((double)y2[i] - a2);
+    if (k > 0) {
+      y1[i] = (T)((double)y1[i] - a1);
+      y2[i] = (T)((double)y2[i] - a2);
+    }
+    sq = fma((double)y2[i], (double)y2[i], sq);
   }
-}
-
-// After the first projection sweep: the norm of the correction's image before (nM) and after it, relative (rel),
-// and whether a second sweep restores orthogonality (1e-5 < rel < 0.5, "twice is enough"; the cancellation bound
-// 1e-5 of OrthonormalizationMultigrid.cs:263-337).  With an empty history there is nothing to project and rel = 1.
-__global__ void ortho_decide1_kernel(OrthoState* s, const double* proj, int* err) {
+  double tot;
+  if (!grid_total(sq, partial, ticket, &tot) || threadIdx.x != 0) return;
+  const double nrm = sqrt(tot);
+  proj[0] = nrm;
+  if (sweep == 2) {
+    s->rel = s->nM > 0.0 ? nrm / s->nM : 0.0;
+    return;
+  }
   const double nM = sqrt(proj[1]);
-  if (!isfinite(nM) || !isfinite(proj[0])) {
+  if (!isfinite(nM) || !isfinite(nrm)) {
     atomicOr(err, kDevErrNaN);
     s->nM = 0.0;
     s->rel = 0.0;
@@ -237,49 +315,69 @@ __global__ void ortho_decide1_kernel(OrthoState* s, const double* proj, int* err
     return;
   }
   s->nM = nM;
-  s->rel = nM > 0.0 ? proj[0] / nM : 0.0;
-  s->second = (s->k > 0 && nM > 0.0 && s->rel > 1e-5 && s->rel < 0.5) ? 1 : 0;
+  s->rel = nM > 0.0 ? nrm / nM : 0.0;
+  s->second = (k > 0 && nM > 0.0 && s->rel > 1e-5 && s->rel < 0.5) ? 1 : 0;
 }
 
-__global__ void ortho_decide2_kernel(OrthoState* s, const double* proj) {
-  s->rel = s->nM > 0.0 ? proj[0] / s->nM : 0.0;
-}
-
-// The correction is kept, normalised by its projected image norm, unless nothing independent of the history is
-// left in it (rel <= 1e-5, or a zero correction); then it is dropped (stored as zero, which projects and minimises
-// to nothing) and the level's post-smoothing loop ends, as after the reference's cancellation branch.
-__global__ void ortho_final_kernel(OrthoState* s, const double* proj) {
-  const bool keep = s->nM > 0.0 && s->rel > 1e-5 && proj[0] > 0.0;
-  s->fac = keep ? 1.0 / proj[0] : 0.0;
-  s->cancel = keep ? 0 : 1;
-}
-
+// The correction is kept, normalised by its projected image norm, unless nothing independent of the history is left in
+// it (rel <= 1e-5, or a zero correction); then it is dropped (stored as zero, which projects and minimises to nothing)
+// and the level's post-smoothing loop ends, as after the reference's cancellation branch.  The normalised correction
+// and image go into history slot k; alpha = <image, Res0>; the last CTA advances k (at most nslots) and decides how
+// MinimizeResidual gets the new residual (RecalcResiPeriod, OrthonormalizationMultigrid.cs:179-190: recompute after a
+// cancellation or every `period` history entries, else update).
 template <typename T>
-__global__ void ortho_store_kernel(const OrthoState* __restrict__ s, T* __restrict__ W, T* __restrict__ MW,
-                                   T* const* __restrict__ sol, T* const* __restrict__ mxx, int nslots, int64_t n,
-                                   int* __restrict__ err) {
+__global__ void __launch_bounds__(kThreads) ortho_commit_kernel(OrthoState* __restrict__ s,
+                                                                const double* __restrict__ proj,
+                                                                const T* __restrict__ W_, const T* __restrict__ MW,
+                                                                T* const* __restrict__ sol, T* const* __restrict__ mxx,
+                                                                int nslots, int period, const T* __restrict__ res0,
+                                                                int64_t n, double* __restrict__ alpha,
+                                                                double* __restrict__ partial,
+                                                                unsigned int* __restrict__ ticket,
+                                                                int* __restrict__ err) {
+  using V = typename V16<T>::type;
+  constexpr int W = V16<T>::W;
   const int k = s->k;
-  if (k < 0 || k >= nslots) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, kDevErrSlots);
-    return;
+  const bool slot_ok = k >= 0 && k < nslots;
+  const bool keep = s->nM > 0.0 && s->rel > 1e-5 && proj[0] > 0.0;
+  const double f = keep ? 1.0 / proj[0] : 0.0;
+  double acc = 0.0;
+  if (slot_ok) {
+    T* S = sol[k];
+    T* M = mxx[k];
+    const int64_t nv = n / W;
+    const int64_t stride = (int64_t)gridDim.x * kThreads;
+    for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < nv; i += stride) {
+      V w = reinterpret_cast<const V*>(W_)[i];
+      V m = reinterpret_cast<const V*>(MW)[i];
+      const V q = reinterpret_cast<const V*>(res0)[i];
+      T* ww = reinterpret_cast<T*>(&w);
+      T* mm = reinterpret_cast<T*>(&m);
+      const T* qq = reinterpret_cast<const T*>(&q);
+#pragma unroll
+      for (int u = 0; u < W; ++u) {
+        ww[u] = (T)((double)ww[u] * f);
+        mm[u] = (T)((double)mm[u] * f);
+        acc = fma((double)mm[u], (double)qq[u], acc);
+      }
+      reinterpret_cast<V*>(S)[i] = w;
+      reinterpret_cast<V*>(M)[i] = m;
+    }
+    for (int64_t i = nv * W + (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += stride) {
+      S[i] = (T)((double)W_[i] * f);
+      const T m = (T)((double)MW[i] * f);
+      M[i] = m;
+      acc = fma((double)m, (double)res0[i], acc);
+    }
   }
-  const double f = s->fac;
-  T* S = sol[k];
-  T* M = mxx[k];
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const T w = (T)((double)W[i] * f);
-    const T mw = (T)((double)MW[i] * f);
-    W[i] = w;
-    MW[i] = mw;
-    S[i] = w;
-    M[i] = mw;
-  }
-}
-
-// RecalcResiPeriod (OrthonormalizationMultigrid.cs:179-190): recompute after a cancellation or every `period`
-// history entries, else update.
-__global__ void ortho_advance_kernel(OrthoState* s, int period, int nslots) {
-  s->k = min(s->k + 1, nslots);
+  double tot;
+  if (!grid_total(acc, partial, ticket, &tot) || threadIdx.x != 0) return;
+  if (!slot_ok) atomicOr(err, kDevErrSlots);
+  *alpha = tot;
+  s->fac = f;
+  s->cancel = keep ? 0 : 1;
+  s->slot = slot_ok ? k : -1;
+  s->k = min(k + 1, nslots);
   const bool rec = period <= 1 || s->cancel != 0 || (s->k % period) == 0;
   s->recalc = rec ? 1 : 0;
   s->update = rec ? 0 : 1;
@@ -287,8 +385,7 @@ __global__ void ortho_advance_kernel(OrthoState* s, int period, int nslots) {
 
 // MinimizeResidual's checks (OrthonormalizationMultigrid.cs:192-209): NaN and residual increase raise in the
 // reference; here they set the error word (the host raises after the graph) and stop the level.
-__global__ void minimize_check_kernel(OrthoState* s, const double* rn_new, TermParams tp, int* err) {
-  const double rn = *rn_new;
+__device__ __forceinline__ void minimize_check(OrthoState* s, double rn, const TermParams& tp, int* err) {
   const double old = s->rn;
   s->rn = rn;
   if (!isfinite(rn)) {
@@ -305,6 +402,86 @@ __global__ void minimize_check_kernel(OrthoState* s, const double* rn_new, TermP
   if (s->active) s->active = term_continue(tp, s->iter, s->r0, rn) ? 1 : 0;
 }
 
+// MinimizeResidual with the correction and image of the current history slot: X += alpha S and, when the residual is
+// updated (s->update), Res -= alpha M, |Res| and the checks.
+template <typename T>
+__global__ void __launch_bounds__(kThreads) ortho_minimize_kernel(OrthoState* __restrict__ s,
+                                                                  T* const* __restrict__ sol,
+                                                                  T* const* __restrict__ mxx,
+                                                                  const double* __restrict__ alpha, T* __restrict__ x,
+                                                                  T* __restrict__ res, int64_t n, TermParams tp,
+                                                                  double* __restrict__ partial,
+                                                                  unsigned int* __restrict__ ticket,
+                                                                  int* __restrict__ err) {
+  using V = typename V16<T>::type;
+  constexpr int W = V16<T>::W;
+  const int slot = s->slot;
+  const bool upd = s->update != 0;
+  double acc = 0.0;
+  if (slot >= 0) {
+    const double al = *alpha;
+    const T* S = sol[slot];
+    const T* M = mxx[slot];
+    const int64_t nv = n / W;
+    const int64_t stride = (int64_t)gridDim.x * kThreads;
+    for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < nv; i += stride) {
+      const V u = reinterpret_cast<const V*>(S)[i];
+      V v = reinterpret_cast<V*>(x)[i];
+      const T* uu = reinterpret_cast<const T*>(&u);
+      T* vv = reinterpret_cast<T*>(&v);
+#pragma unroll
+      for (int w = 0; w < W; ++w) vv[w] = (T)((double)vv[w] + al * (double)uu[w]);
+      reinterpret_cast<V*>(x)[i] = v;
+      if (upd) {
+        const V m = reinterpret_cast<const V*>(M)[i];
+        V r = reinterpret_cast<V*>(res)[i];
+        const T* mm = reinterpret_cast<const T*>(&m);
+        T* rr = reinterpret_cast<T*>(&r);
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          rr[w] = (T)((double)rr[w] - al * (double)mm[w]);
+          acc = fma((double)rr[w], (double)rr[w], acc);
+        }
+        reinterpret_cast<V*>(res)[i] = r;
+      }
+    }
+    for (int64_t i = nv * W + (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += stride) {
+      x[i] = (T)((double)x[i] + al * (double)S[i]);
+      if (upd) {
+        const T r = (T)((double)res[i] - al * (double)M[i]);
+        res[i] = r;
+        acc = fma((double)r, (double)r, acc);
+      }
+    }
+  }
+  if (!upd) return;
+  double tot;
+  if (grid_total(acc, partial, ticket, &tot) && threadIdx.x == 0) minimize_check(s, sqrt(tot), tp, err);
+}
+
+// |Res| and the checks after a recomputed residual (s->recalc)
+template <typename T>
+__global__ void __launch_bounds__(kThreads) ortho_check_kernel(OrthoState* __restrict__ s, const T* __restrict__ res,
+                                                               int64_t n, TermParams tp,
+                                                               double* __restrict__ partial,
+                                                               unsigned int* __restrict__ ticket,
+                                                               int* __restrict__ err) {
+  using V = typename V16<T>::type;
+  constexpr int W = V16<T>::W;
+  if (s->recalc == 0) return;
+  const int64_t nv = n / W;
+  const int64_t stride = (int64_t)gridDim.x * kThreads;
+  double acc = 0.0;
+  for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < nv; i += stride) {
+    const V r = reinterpret_cast<const V*>(res)[i];
+    acc += vdot(r, r);
+  }
+  for (int64_t i = nv * W + (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += stride)
+    acc = fma((double)res[i], (double)res[i], acc);
+  double tot;
+  if (grid_total(acc, partial, ticket, &tot) && threadIdx.x == 0) minimize_check(s, sqrt(tot), tp, err);
+}
+
 __global__ void level_begin_kernel(OrthoState* s, const double* r0_in, TermParams tp) {
   const double r0 = *r0_in;
   s->k = 0;
@@ -313,6 +490,7 @@ __global__ void level_begin_kernel(OrthoState* s, const double* r0_in, TermParam
   s->recalc = 1;
   s->update = 0;
   s->restart = 0;
+  s->slot = -1;
   s->iter = 1;
   s->iterations = 0;
   s->r0 = r0;
@@ -538,32 +716,63 @@ int grid_for(int64_t n_work) {
 
 template <typename T>
 void hist_dots_impl(HistScratch& s, const T* const* hist, const int* k, const T* m, int64_t n, double* beta,
-                    double* self, cudaStream_t st) {
+                    double* self, cudaStream_t st, const int* active) {
   require(s.chunks > 0, "history multi-dot: scratch not initialised");
   const int W = 16 / (int)sizeof(T);
   const int G = std::min(grid_for(std::max<int64_t>(n / W, 1)), s.grid);
   require((reinterpret_cast<uintptr_t>(m) & 15) == 0, "history multi-dot: unaligned vector");
   hist_dots_kernel<T><<<dim3(G, s.chunks), kThreads, 0, st>>>(hist, k, s.chunks * kChunk > s.slots ? s.slots : s.chunks * kChunk,
-                                                                m, n, beta, self, s.partial.p, s.ticket.p);
+                                                                m, n, beta, self, s.partial.p, s.ticket.p, active);
   BSGPU_CHECK_LAUNCH();
 }
 
 template <typename T>
-void hist_axpy2_impl(const T* const* x1, const T* const* x2, const int* k, int kmax, const double* beta, T* y1, T* y2,
-                     int64_t n, cudaStream_t st) {
+bool aligned16(std::initializer_list<const T*> v) {
+  for (const T* p : v)
+    if (reinterpret_cast<uintptr_t>(p) & 15) return false;
+  return true;
+}
+
+// grid of the fused level kernels: one CTA per 256 16-byte pieces, at most four per SM (their totals end on one ticket)
+template <typename T>
+int level_grid(const HistScratch& s, int64_t n) {
   const int W = 16 / (int)sizeof(T);
-  require((reinterpret_cast<uintptr_t>(y1) & 15) == 0 && (reinterpret_cast<uintptr_t>(y2) & 15) == 0,
-          "history multi-axpy: unaligned vector");
-  require(kmax >= 1 && kmax <= kHistMax, "history multi-axpy: 1 <= slots <= 128");
-  hist_axpy2_kernel<T><<<grid_for(std::max<int64_t>(n / W, 1)) * 2, kThreads, 0, st>>>(x1, x2, k, kmax, beta, y1, y2,
-                                                                                       n);
+  return (int)std::max<int64_t>(1, std::min<int64_t>((n / W + kThreads - 1) / kThreads, 2 * (int64_t)s.grid));
+}
+
+template <typename T>
+void project_impl(HistScratch& h, const T* const* x1, const T* const* x2, OrthoState* s, int sweep,
+                  const double* beta, T* y1, T* y2, int64_t n, double* proj, int* err, cudaStream_t st) {
+  require(aligned16<T>({y1, y2}), "ortho_project: unaligned vector");
+  ortho_project_kernel<T><<<level_grid<T>(h, n), kThreads, 0, st>>>(x1, x2, s, h.slots, sweep, beta, y1, y2, n, proj,
+                                                                    h.total.p, h.ticket.p + h.chunks, err);
   BSGPU_CHECK_LAUNCH();
 }
 
 template <typename T>
-void store_impl(OrthoState* s, T* W, T* MW, T* const* sol, T* const* mxx, int nslots, int64_t n, int* err,
-                cudaStream_t st) {
-  ortho_store_kernel<T><<<grid_for(n) * 4, kThreads, 0, st>>>(s, W, MW, sol, mxx, nslots, n, err);
+void commit_impl(HistScratch& h, OrthoState* s, const double* proj, const T* W, const T* MW, T* const* sol,
+                 T* const* mxx, int nslots, int period, const T* res0, int64_t n, double* alpha, int* err,
+                 cudaStream_t st) {
+  require(aligned16<T>({W, MW, res0}), "ortho_commit: unaligned vector");
+  ortho_commit_kernel<T><<<level_grid<T>(h, n), kThreads, 0, st>>>(s, proj, W, MW, sol, mxx, nslots, period, res0, n,
+                                                                   alpha, h.total.p, h.ticket.p + h.chunks, err);
+  BSGPU_CHECK_LAUNCH();
+}
+
+template <typename T>
+void minimize_impl(HistScratch& h, OrthoState* s, T* const* sol, T* const* mxx, const double* alpha, T* x, T* res,
+                   int64_t n, TermParams tp, int* err, cudaStream_t st) {
+  require(aligned16<T>({x, res}), "ortho_minimize: unaligned vector");
+  ortho_minimize_kernel<T><<<level_grid<T>(h, n), kThreads, 0, st>>>(s, sol, mxx, alpha, x, res, n, tp, h.total.p,
+                                                                     h.ticket.p + h.chunks, err);
+  BSGPU_CHECK_LAUNCH();
+}
+
+template <typename T>
+void check_impl(HistScratch& h, OrthoState* s, const T* res, int64_t n, TermParams tp, int* err, cudaStream_t st) {
+  require(aligned16<T>({res}), "ortho_check: unaligned vector");
+  ortho_check_kernel<T><<<level_grid<T>(h, n), kThreads, 0, st>>>(s, res, n, tp, h.total.p, h.ticket.p + h.chunks,
+                                                                  err);
   BSGPU_CHECK_LAUNCH();
 }
 
@@ -575,14 +784,15 @@ void copy_if_impl(const T* x, T* y, int64_t n, const int* flag, cudaStream_t st)
 
 }  // namespace
 
-void HistScratch::init(int cap) {
+void HistScratch::init(int cap, cudaStream_t st) {
   require(cap >= 1 && cap <= kHistMax, "history length must be in 1..128");
   slots = cap;
   chunks = (cap + kChunk - 1) / kChunk;
   grid = num_sms() * 2;
   partial.alloc((size_t)chunks * kProducts * grid);
-  ticket.alloc(chunks);
-  BSGPU_CUDA(cudaMemset(ticket.p, 0, chunks * sizeof(unsigned int)));
+  ticket.alloc(chunks + 1);
+  BSGPU_CUDA(cudaMemsetAsync(ticket.p, 0, (chunks + 1) * sizeof(unsigned int), st));
+  total.alloc(2 * (size_t)grid);
 }
 
 void cond_set(cudaGraphConditionalHandle h, const int* a, const int* not_b, const int* k, int cap, unsigned int* exec,
@@ -597,50 +807,35 @@ void positive_flag(const double* x, int* flag, cudaStream_t st) {
 }
 
 void hist_dots(HistScratch& s, const double* const* hist, const int* k, const double* m, int64_t n, double* beta,
-               double* self, cudaStream_t st) {
-  hist_dots_impl<double>(s, hist, k, m, n, beta, self, st);
+               double* self, cudaStream_t st, const int* active) {
+  hist_dots_impl<double>(s, hist, k, m, n, beta, self, st, active);
 }
 void hist_dots(HistScratch& s, const float* const* hist, const int* k, const float* m, int64_t n, double* beta,
-               double* self, cudaStream_t st) {
-  hist_dots_impl<float>(s, hist, k, m, n, beta, self, st);
+               double* self, cudaStream_t st, const int* active) {
+  hist_dots_impl<float>(s, hist, k, m, n, beta, self, st, active);
 }
-void hist_axpy2(const double* const* x1, const double* const* x2, const int* k, int kmax, const double* beta,
-                double* y1, double* y2, int64_t n, cudaStream_t st) {
-  hist_axpy2_impl<double>(x1, x2, k, kmax, beta, y1, y2, n, st);
-}
-void hist_axpy2(const float* const* x1, const float* const* x2, const int* k, int kmax, const double* beta, float* y1,
-                float* y2, int64_t n, cudaStream_t st) {
-  hist_axpy2_impl<float>(x1, x2, k, kmax, beta, y1, y2, n, st);
-}
+#define BSGPU_LEVEL(T)                                                                                               \
+  void ortho_project(HistScratch& h, const T* const* x1, const T* const* x2, OrthoState* s, int sweep,               \
+                     const double* beta, T* y1, T* y2, int64_t n, double* proj, int* err, cudaStream_t st) {         \
+    project_impl<T>(h, x1, x2, s, sweep, beta, y1, y2, n, proj, err, st);                                            \
+  }                                                                                                                  \
+  void ortho_commit(HistScratch& h, OrthoState* s, const double* proj, const T* W, const T* MW, T* const* sol,       \
+                    T* const* mxx, int nslots, int period, const T* res0, int64_t n, double* alpha, int* err,        \
+                    cudaStream_t st) {                                                                               \
+    commit_impl<T>(h, s, proj, W, MW, sol, mxx, nslots, period, res0, n, alpha, err, st);                            \
+  }                                                                                                                  \
+  void ortho_minimize(HistScratch& h, OrthoState* s, T* const* sol, T* const* mxx, const double* alpha, T* x,        \
+                      T* res, int64_t n, TermParams tp, int* err, cudaStream_t st) {                                 \
+    minimize_impl<T>(h, s, sol, mxx, alpha, x, res, n, tp, err, st);                                                 \
+  }                                                                                                                  \
+  void ortho_check(HistScratch& h, OrthoState* s, const T* res, int64_t n, TermParams tp, int* err,                  \
+                   cudaStream_t st) {                                                                                \
+    check_impl<T>(h, s, res, n, tp, err, st);                                                                        \
+  }
+BSGPU_LEVEL(double)
+BSGPU_LEVEL(float)
+#undef BSGPU_LEVEL
 
-void ortho_decide1(OrthoState* s, const double* proj, int* err, cudaStream_t st) {
-  ortho_decide1_kernel<<<1, 1, 0, st>>>(s, proj, err);
-  BSGPU_CHECK_LAUNCH();
-}
-void ortho_decide2(OrthoState* s, const double* proj, cudaStream_t st) {
-  ortho_decide2_kernel<<<1, 1, 0, st>>>(s, proj);
-  BSGPU_CHECK_LAUNCH();
-}
-void ortho_final(OrthoState* s, const double* proj, cudaStream_t st) {
-  ortho_final_kernel<<<1, 1, 0, st>>>(s, proj);
-  BSGPU_CHECK_LAUNCH();
-}
-void ortho_store(OrthoState* s, double* W, double* MW, double* const* sol, double* const* mxx, int nslots, int64_t n,
-                 int* err, cudaStream_t st) {
-  store_impl<double>(s, W, MW, sol, mxx, nslots, n, err, st);
-}
-void ortho_store(OrthoState* s, float* W, float* MW, float* const* sol, float* const* mxx, int nslots, int64_t n,
-                 int* err, cudaStream_t st) {
-  store_impl<float>(s, W, MW, sol, mxx, nslots, n, err, st);
-}
-void ortho_advance(OrthoState* s, int period, int nslots, cudaStream_t st) {
-  ortho_advance_kernel<<<1, 1, 0, st>>>(s, period, nslots);
-  BSGPU_CHECK_LAUNCH();
-}
-void minimize_check(OrthoState* s, const double* rn_new, TermParams tp, int* err, cudaStream_t st) {
-  minimize_check_kernel<<<1, 1, 0, st>>>(s, rn_new, tp, err);
-  BSGPU_CHECK_LAUNCH();
-}
 void level_begin(OrthoState* s, const double* r0_in, TermParams tp, cudaStream_t st) {
   level_begin_kernel<<<1, 1, 0, st>>>(s, r0_in, tp);
   BSGPU_CHECK_LAUNCH();

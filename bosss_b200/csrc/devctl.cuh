@@ -27,7 +27,7 @@ struct OrthoState {
   int active;   // the level keeps iterating (termination test)
   int iter;     // iteration number, 1-based (iIter of the reference loop)
   int iterations;  // completed iterations (ThisLevelIterations)
-  int pad;
+  int slot;     // history slot of the last correction
   double nM;    // |A x| of the new correction before projection
   double rel;   // |A x| after projection, relative to nM
   double fac;   // scaling of the stored correction (1/|A x| after projection; 0 = dropped)
@@ -51,37 +51,41 @@ void positive_flag(const double* x, int* flag, cudaStream_t st);
 // one launch.  scratch: partial sums and tickets sized by hist_dots_scratch.
 struct HistScratch {
   DBuf<double> partial;
-  DBuf<unsigned int> ticket;
+  DBuf<unsigned int> ticket;  // one per chunk, and one for the level's one-value totals
+  DBuf<double> total;         // their partial sums
   int grid = 0, chunks = 0, slots = 0;  // slots: entries of the pointer arrays (*k is clamped to it)
-  void init(int cap);
+  void init(int cap, cudaStream_t st);
 };
 void hist_dots(HistScratch& s, const double* const* hist, const int* k, const double* m, int64_t n, double* beta,
-               double* self, cudaStream_t st);
+               double* self, cudaStream_t st, const int* active = nullptr);
 void hist_dots(HistScratch& s, const float* const* hist, const int* k, const float* m, int64_t n, double* beta,
-               double* self, cudaStream_t st);
-// y1 -= sum_{j<*k} beta[j] x1[j], y2 -= sum_{j<*k} beta[j] x2[j]; one launch (*k clamped to kmax <= kHistMax,
-// the entries of the pointer arrays).
+               double* self, cudaStream_t st, const int* active = nullptr);
 constexpr int kHistMax = 128;
-void hist_axpy2(const double* const* x1, const double* const* x2, const int* k, int kmax, const double* beta,
-                double* y1, double* y2, int64_t n, cudaStream_t st);
-void hist_axpy2(const float* const* x1, const float* const* x2, const int* k, int kmax, const double* beta, float* y1,
-                float* y2, int64_t n, cudaStream_t st);
 // upper bound on the iterations of any recorded loop (a safety bound above every configured limit)
 constexpr int kMaxRecordedIterations = 100000;
 
-// AddSol decisions.  proj[0] = |M| after the sweep, proj[1] = |M|^2 before the first sweep.
-void ortho_decide1(OrthoState* s, const double* proj, int* err, cudaStream_t st);
-void ortho_decide2(OrthoState* s, const double* proj, cudaStream_t st);
-void ortho_final(OrthoState* s, const double* proj, cudaStream_t st);
-// W *= fac, MW *= fac, and the two stored into history slot *k (slots: device arrays of nslots pointers)
-void ortho_store(OrthoState* s, double* W, double* MW, double* const* sol, double* const* mxx, int nslots, int64_t n,
-                 int* err, cudaStream_t st);
-void ortho_store(OrthoState* s, float* W, float* MW, float* const* sol, float* const* mxx, int nslots, int64_t n,
-                 int* err, cudaStream_t st);
-// k += 1 (at most nslots) and the residual period decision of the following MinimizeResidual
-void ortho_advance(OrthoState* s, int period, int nslots, cudaStream_t st);
-// MinimizeResidual's checks on the new residual norm rn_new and the termination test of the level
-void minimize_check(OrthoState* s, const double* rn_new, TermParams tp, int* err, cudaStream_t st);
+// AddSol and MinimizeResidual in four launches after the image MW = A W of a new correction W and its projections
+// beta (hist_dots, with proj[1] = |MW|^2):
+//   ortho_project   W, MW -= history * beta, |MW| into proj[0], the re-orthonormalisation test (sweep 1; sweep 2 runs
+//                   only where the test asked for it, as does a hist_dots with &s->second);
+//   ortho_commit    the normalised correction and image into history slot k, alpha = <image, res0>, k += 1, the
+//                   residual period decision;
+//   ortho_minimize  x += alpha S and, when the residual is updated, res -= alpha M with |res|, the checks and the
+//                   termination test;
+//   ortho_check     the same checks after a recomputed residual (s->recalc; the product in between is the caller's).
+// sol, mxx: device arrays of the history's vectors (16-byte aligned).
+#define BSGPU_LEVEL(T)                                                                                               \
+  void ortho_project(HistScratch& h, const T* const* x1, const T* const* x2, OrthoState* s, int sweep,               \
+                     const double* beta, T* y1, T* y2, int64_t n, double* proj, int* err, cudaStream_t st);          \
+  void ortho_commit(HistScratch& h, OrthoState* s, const double* proj, const T* W, const T* MW, T* const* sol,       \
+                    T* const* mxx, int nslots, int period, const T* res0, int64_t n, double* alpha, int* err,        \
+                    cudaStream_t st);                                                                                \
+  void ortho_minimize(HistScratch& h, OrthoState* s, T* const* sol, T* const* mxx, const double* alpha, T* x,        \
+                      T* res, int64_t n, TermParams tp, int* err, cudaStream_t st);                                  \
+  void ortho_check(HistScratch& h, OrthoState* s, const T* res, int64_t n, TermParams tp, int* err, cudaStream_t st);
+BSGPU_LEVEL(double)
+BSGPU_LEVEL(float)
+#undef BSGPU_LEVEL
 // start of a level solve: r0 = rn = *r0_in, k = 0, iter = 1, iterations = 0, active = term(1, r0, r0)
 void level_begin(OrthoState* s, const double* r0_in, TermParams tp, cudaStream_t st);
 // start of an iteration: restart = (k >= cap) (then k = 0), cancel = 0

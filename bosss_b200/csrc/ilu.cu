@@ -180,7 +180,8 @@ void apply_impl(IluApply& a, const T* vals, const T* uinv, const T* b, T* x, int
 
 }  // namespace
 
-void IluApply::init(const Matrix& M_, const std::vector<int64_t>& lptr, const std::vector<int32_t>& order_) {
+void IluApply::init(const Matrix& M_, const std::vector<int64_t>& lptr, const std::vector<int32_t>& order_,
+                    cudaStream_t st) {
   M = &M_;
   const int64_t nb = M->nb;
   if (nb == 0) return;
@@ -203,13 +204,13 @@ void IluApply::init(const Matrix& M_, const std::vector<int64_t>& lptr, const st
   for (int64_t i = 0; i < nb; ++i) back[at[lev[i]]++] = (int32_t)i;
   order.alloc(nb);
   rorder.alloc(nb);
-  BSGPU_CUDA(cudaMemcpy(rorder.p, back.data(), nb * 4, cudaMemcpyHostToDevice));
+  BSGPU_CUDA(cudaMemcpyAsync(rorder.p, back.data(), nb * 4, cudaMemcpyHostToDevice, st));
   diag.alloc(nb);
-  BSGPU_CUDA(cudaMemcpy(order.p, order_.data(), nb * 4, cudaMemcpyHostToDevice));
-  BSGPU_CUDA(cudaMemcpy(diag.p, d.data(), nb * 8, cudaMemcpyHostToDevice));
+  BSGPU_CUDA(cudaMemcpyAsync(order.p, order_.data(), nb * 4, cudaMemcpyHostToDevice, st));
+  BSGPU_CUDA(cudaMemcpyAsync(diag.p, d.data(), nb * 8, cudaMemcpyHostToDevice, st));
   const size_t words = M->single ? 1 : 2;
   state.alloc(3);
-  BSGPU_CUDA(cudaMemset(state.p, 0, 3 * sizeof(unsigned int)));
+  BSGPU_CUDA(cudaMemsetAsync(state.p, 0, 3 * sizeof(unsigned int), st));
   // warps for two of the widest wavefronts: while one is being computed the blocks of the next are on their way
   int64_t widest = 1;
   for (size_t l = 0; l + 1 < lptr.size(); ++l) widest = std::max(widest, lptr[l + 1] - lptr[l]);
@@ -224,7 +225,7 @@ void IluApply::init(const Matrix& M_, const std::vector<int64_t>& lptr, const st
   require(per_sm >= 1, "ILU: the kernel does not fit the device", BSGPU_ERR_UNSUPPORTED);
   grid = (int)std::min<int64_t>((2 * widest + kWarps - 1) / kWarps, (int64_t)per_sm * num_sms());
   packets.alloc((2 * (size_t)M->N + (size_t)grid * kWarps * M->Np) * words);
-  BSGPU_CUDA(cudaMemset(packets.p, 0, packets.bytes()));
+  BSGPU_CUDA(cudaMemsetAsync(packets.p, 0, packets.bytes(), st));
 }
 
 void ilu_apply(IluApply& a, const double* uinv, const double* b, double* x, int* err, int err_bit, cudaStream_t st) {

@@ -12,7 +12,8 @@ struct IluApply {
   DBuf<unsigned int> state;       // epoch, failure, exits
   int grid = 0;
   // lptr: offsets of the wavefronts in `order`
-  void init(const Matrix& M_, const std::vector<int64_t>& lptr, const std::vector<int32_t>& order_);
+  void init(const Matrix& M_, const std::vector<int64_t>& lptr, const std::vector<int32_t>& order_,
+            cudaStream_t st);
 };
 
 // x = U^{-1} L^{-1} b; uinv: inverses of U's diagonal blocks, column-major at diag_offsets(M).  err gets `err_bit`

@@ -941,7 +941,7 @@ void run_impl(PcgLaunch& l, const ST* vals, const PcgCall<T>& c, cudaStream_t st
 
 // The small kernel with the widest split of the rows that still gives every CTA one tile, on at most one CTA per SM.
 template <typename T, typename ST>
-bool init_small(PcgLaunch& l) {
+bool init_small(PcgLaunch& l, cudaStream_t st) {
   const Matrix& A = *l.A;
   for (int w : {4, 2, 1}) {
     const bool ok = pick_small<T, ST>(A, w, [&](auto tag) {
@@ -956,7 +956,7 @@ bool init_small(PcgLaunch& l) {
     l.kind = PcgLaunch::kSmall;
     l.split = w;
     l.packets.alloc(6 * (size_t)l.grid + (size_t)A.N * sizeof(T) / 4);
-    BSGPU_CUDA(cudaMemset(l.packets.p, 0, l.packets.bytes()));
+    BSGPU_CUDA(cudaMemsetAsync(l.packets.p, 0, l.packets.bytes(), st));
     return true;
   }
   return false;
@@ -985,26 +985,26 @@ bool init_large(PcgLaunch& l) {
 }
 
 template <typename T, typename ST>
-bool init_impl(PcgLaunch& l) {
-  if (!init_small<T, ST>(l) && !init_large<T, ST>(l)) return false;
+bool init_impl(PcgLaunch& l, cudaStream_t st) {
+  if (!init_small<T, ST>(l, st) && !init_large<T, ST>(l)) return false;
   l.bar.alloc(3);
-  BSGPU_CUDA(cudaMemset(l.bar.p, 0, 3 * sizeof(unsigned int)));
+  BSGPU_CUDA(cudaMemsetAsync(l.bar.p, 0, 3 * sizeof(unsigned int), st));
   return true;
 }
 
 }  // namespace
 
 template <typename T>
-bool PcgLaunch::init(const Matrix& A_) {
+bool PcgLaunch::init(const Matrix& A_, cudaStream_t st) {
   A = &A_;
   if (A->N == 0) return false;
   if constexpr (sizeof(T) == 4) {
-    if (A->half) return init_impl<float, __half>(*this);
+    if (A->half) return init_impl<float, __half>(*this, st);
   }
-  return init_impl<T, T>(*this);
+  return init_impl<T, T>(*this, st);
 }
-template bool PcgLaunch::init<double>(const Matrix&);
-template bool PcgLaunch::init<float>(const Matrix&);
+template bool PcgLaunch::init<double>(const Matrix&, cudaStream_t);
+template bool PcgLaunch::init<float>(const Matrix&, cudaStream_t);
 
 void pcg_run(PcgLaunch& l, const PcgCall<double>& c, cudaStream_t st) {
   require(!l.A->single, "precision mismatch");

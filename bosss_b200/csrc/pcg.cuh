@@ -31,7 +31,7 @@ struct PcgLaunch {
   DBuf<unsigned int> bar;     // arrivals (or the epoch of the packets), failure, exits
   // false: the matrix is served by separate launches (too large, or no kernel for its layout)
   template <typename T>
-  bool init(const Matrix& A_);
+  bool init(const Matrix& A_, cudaStream_t st);
 };
 
 // One call of the solver: x <- solution of A x = b (x: initial guess, known to be zero with `zero`), z = Dinv r with

@@ -42,6 +42,7 @@ Ctx::Ctx() {
   BSGPU_CUDA(cudaMemset(dflag.p, 0, 256 * sizeof(int)));
   BSGPU_CUDA(cudaMemset(dscal.p, 0, scal_cap * sizeof(double)));
   red.init();
+  BSGPU_CUDA(cudaStreamSynchronize(nullptr));  // st does not wait for the legacy stream's copies and fills
 }
 Ctx::~Ctx() {
   if (hscal) cudaFreeHost(hscal);
@@ -63,6 +64,7 @@ void Ctx::graph_init() {
   d_exec.alloc(kMaxBodies);
   BSGPU_CUDA(cudaMemset(d_exec.p, 0, kMaxBodies * sizeof(unsigned int)));
   h_exec.assign(kMaxBodies, 0);
+  BSGPU_CUDA(cudaStreamSynchronize(nullptr));
   for (int i = 0; i < kMaxDepth; ++i) {
     cudaStream_t b = nullptr;
     BSGPU_CUDA(cudaStreamCreateWithFlags(&b, cudaStreamNonBlocking));
@@ -310,6 +312,7 @@ int elt_grid(int64_t n) {
 template <typename T>
 struct BlockJacobiT : Solver<T> {
   bool graphable() const override { return true; }
+  bool overwrites() const override { return updates > 0; }
   const Matrix* A;
   DBuf<T> dinv;
   DBuf<T> tmp;
@@ -357,6 +360,7 @@ struct BlockJacobiT : Solver<T> {
 template <typename T>
 struct BlockGST : Solver<T> {
   bool graphable() const override { return true; }
+  bool overwrites() const override { return true; }
   const Matrix* A;
   DBuf<T> dinv;
   std::vector<DBuf<int32_t>> rows;
@@ -402,6 +406,7 @@ struct BlockGST : Solver<T> {
 template <typename T>
 struct ILU0T : Solver<T> {
   bool graphable() const override { return true; }
+  bool overwrites() const override { return true; }
   std::unique_ptr<Matrix> M64, M32;
   const Matrix* M = nullptr;
   DBuf<T> uinv;
@@ -463,6 +468,7 @@ struct ILU0T : Solver<T> {
 template <typename T>
 struct ILUNaturalT : Solver<T> {
   bool graphable() const override { return true; }
+  bool overwrites() const override { return true; }
   std::unique_ptr<Matrix> M64, M32;
   const Matrix* M = nullptr;
   DBuf<double> uinv64;
@@ -476,7 +482,7 @@ struct ILUNaturalT : Solver<T> {
     std::vector<int64_t> lptr;
     ilu_wavefronts(*A64, lptr, order);
     DBuf<int32_t> rows(std::max<int64_t>(nb, 1));
-    if (nb) BSGPU_CUDA(cudaMemcpy(rows.p, order.data(), nb * 4, cudaMemcpyHostToDevice));
+    if (nb) BSGPU_CUDA(cudaMemcpyAsync(rows.p, order.data(), nb * 4, cudaMemcpyHostToDevice, c.st));
     const std::vector<int64_t> o = diag_offsets(*A64);
     uinv64.alloc(std::max<int64_t>(o.back(), 1));
     if constexpr (sizeof(T) == 4) uinv32.alloc(std::max<int64_t>(o.back(), 1));
@@ -493,7 +499,7 @@ struct ILUNaturalT : Solver<T> {
     } else {
       M = M64.get();
     }
-    apply.init(*M, lptr, order);
+    apply.init(*M, lptr, order, c.st);
     c.graph_init();  // the error word
   }
   const T* uinv() const {
@@ -519,6 +525,7 @@ struct ILUNaturalT : Solver<T> {
 template <typename T>
 struct SchwarzT : Solver<T> {
   bool graphable() const override { return true; }
+  bool overwrites() const override { return updates > 0; }
   const Matrix* A;
   std::unique_ptr<Matrix> M;
   DBuf<T> r;
@@ -554,6 +561,7 @@ struct SchwarzT : Solver<T> {
 template <typename T>
 struct BlockSchwarzT : Solver<T> {
   bool graphable() const override { return true; }
+  bool overwrites() const override { return true; }
   const Matrix* A;
   std::unique_ptr<SchwarzBlocks> S;
   DBuf<T> r;
@@ -652,7 +660,7 @@ struct PCGT : Solver<T> {
         invert_diag_blocks(*A64, nullptr, dinv.p, err, c.st);
       c.check_flag(err, "PCG: singular diagonal block");
     }
-    persistent = launch.init<T>(*A);
+    persistent = launch.init<T>(*A, c.st);
     if (!persistent) {
       active = c.flag();
       c.tune(*A, 0);
@@ -859,17 +867,21 @@ struct PCGT : Solver<T> {
 // ---------------------------------------------------------------------------------------------------------------
 template <typename T>
 struct OrthoT {
+  static constexpr int kStateScalars = sizeof(OrthoState) / sizeof(double);
+  static_assert(sizeof(OrthoState) % sizeof(double) == 0, "the state is fetched as doubles");
   const Matrix* A;
   int64_t N;
   std::vector<DBuf<T>> Sol, Mxx;
   int k = 0;
   int cap = 96;
+  double* d_state;  // OrthoState of the device-side decisions (devctl.cuh), directly before d_proj: one fetch
   double* d_proj;   // [0] |M| after a projection sweep, [1] |M|^2 before it, [2..] projection coefficients
   double* d_beta;   // = d_proj + 2
   double* d_norm;   // [2]
   double* d_alpha;  // [1]
   bool cancellation = false;
   OrthoT(Ctx& c, const Matrix* A_) : A(A_), N(A_->N) {
+    d_state = c.scal(kStateScalars);
     d_proj = c.scal(kMaxDots + 2);
     d_beta = d_proj + 2;
     d_norm = c.scal(2);
@@ -1040,7 +1052,9 @@ struct OrthoT {
       const T* mx[1] = {Mxx[i].p};
       axpys(1, d_alpha, nullptr, -1.0, mx, Res, N, c.st);
     }
-    const double rn = norm(c, Res);
+    return checked_residual(norm(c, Res), oldN);
+  }
+  static double checked_residual(double rn, double oldN) {
     if (!std::isfinite(rn)) throw Error(BSGPU_ERR_ARITHMETIC, "Orthonormalization: residual is NaN/Inf");
     const double tol = std::max(std::max(rn, oldN) * 0.2, 1.0e-7);
     if (rn > oldN + tol) throw Error(BSGPU_ERR_ARITHMETIC, "Orthonormalization: residual increase");
@@ -1049,84 +1063,108 @@ struct OrthoT {
 
   // ---- recorded form (graph capture): the history length lives on the device ----------------------------------
   // A new correction is built in the fixed buffers W (correction) and MW (its image), projected against the
-  // history by the device-count kernels, normalised and copied into history slot k; MinimizeResidual then uses
-  // W and MW.  A correction with nothing independent of the history left is stored as zero (devctl.cu).
+  // history by the device-count kernels and normalised into history slot k, which MinimizeResidual then uses.
+  // A correction with nothing independent of the history left is stored as zero (devctl.cu).
   int nslots = 0;
   DBuf<T> W, MW;
   DBuf<T*> d_sol, d_mxx;
-  DBuf<OrthoState> state;
   HistScratch hs;
   double* d_hbeta = nullptr;  // projection coefficients of the recorded form [nslots]
-  double* d_rn = nullptr;     // residual norm after MinimizeResidual
-  OrthoState* dev() { return state.p; }
+  OrthoState* dev() { return reinterpret_cast<OrthoState*>(d_state); }
   std::string tag;  // owner's trace name, for the graph statistics
-  void prepare_dev(Ctx& c, int slots) {
-    slots = std::max(1, std::min(slots, cap));
-    require(slots <= kHistMax, "recorded OrthoMG: history longer than 128", BSGPU_ERR_UNSUPPORTED);
-    if (nslots >= slots) return;
+  // fixed buffers and tables for the whole capacity, made once (recordings keep their addresses)
+  void alloc_dev(Ctx& c) {
+    if (W.p) return;
+    require(cap <= kHistMax, "OrthoMG: history longer than 128", BSGPU_ERR_UNSUPPORTED);
+    const int room = std::min(cap + 1, kHistMax);
     W.alloc(std::max<int64_t>(N, 1));
     MW.alloc(std::max<int64_t>(N, 1));
-    while ((int)Sol.size() < slots) {
-      Sol.emplace_back(std::max<int64_t>(N, 1));
-      Mxx.emplace_back(std::max<int64_t>(N, 1));
-    }
-    std::vector<T*> ps(slots), pm(slots);
-    for (int j = 0; j < slots; ++j) {
-      ps[j] = Sol[j].p;
-      pm[j] = Mxx[j].p;
-    }
-    d_sol.alloc(slots);
-    d_mxx.alloc(slots);
-    BSGPU_CUDA(cudaMemcpy(d_sol.p, ps.data(), slots * sizeof(T*), cudaMemcpyHostToDevice));
-    BSGPU_CUDA(cudaMemcpy(d_mxx.p, pm.data(), slots * sizeof(T*), cudaMemcpyHostToDevice));
-    if (!state.p) {
-      state.alloc(1);
-      BSGPU_CUDA(cudaMemset(state.p, 0, sizeof(OrthoState)));
-      d_rn = c.scal(1);
-    }
-    hs.init(slots);
-    d_hbeta = c.scal(slots);
-    nslots = slots;
+    d_sol.alloc(room);
+    d_mxx.alloc(room);
+    hs.init(room, c.st);
+    d_hbeta = c.scal(room);
   }
-  T* next_sol_dev(Ctx& c) {
-    fill(T(0), W.p, N, c.st);
-    return W.p;
+  // the first n history slots exist (the vectors are allocated as the history grows)
+  void need_slots(Ctx& c, int n) {
+    for (; tabled < n; ++tabled) {
+      if ((int)Sol.size() <= tabled) {
+        Sol.emplace_back(std::max<int64_t>(N, 1));
+        Mxx.emplace_back(std::max<int64_t>(N, 1));
+      }
+      // on the solver's stream: the kernels that read the entry come after it
+      BSGPU_CUDA(cudaMemcpyAsync(d_sol.p + tabled, &Sol[tabled].p, sizeof(T*), cudaMemcpyHostToDevice, c.st));
+      BSGPU_CUDA(cudaMemcpyAsync(d_mxx.p + tabled, &Mxx[tabled].p, sizeof(T*), cudaMemcpyHostToDevice, c.st));
+    }
   }
-  // one projection sweep of (W, MW) against the first k history entries; |MW| after it into d_proj[0] and, with
-  // `self`, |MW|^2 before it into d_proj[1]
-  void cgs_dev(Ctx& c, bool self) {
-    hist_dots(hs, d_mxx.p, &state.p->k, MW.p, N, d_hbeta, self ? d_proj + 1 : nullptr, c.st);
-    hist_axpy2(d_sol.p, d_mxx.p, &state.p->k, nslots, d_hbeta, W.p, MW.p, N, c.st);
-    const T* a[1] = {MW.p};
-    dots(c.red, 1, a, a, N, d_proj, 1, c.st);
+  int tabled = 0;  // slots whose vectors are in the pointer tables
+  void prepare_dev(Ctx& c, int slots) {
+    slots = std::max(1, std::min(slots, cap));
+    alloc_dev(c);
+    need_slots(c, slots);
+    nslots = std::max(nslots, slots);
   }
-  void add_sol_dev(Ctx& c) {
+  void add_sol_dev(Ctx& c, const T* Res0, int slots, int* err) {
     spmv(*A, T(1), W.p, T(0), (const T*)nullptr, MW.p, c.st);
-    cgs_dev(c, true);
-    ortho_decide1(state.p, d_proj, c.d_err, c.st);
-    const cudaGraphConditionalHandle h = c.cond_handle();
-    const int body = c.new_body(tag + "second Gram-Schmidt sweep");
-    cond_set(h, &state.p->second, nullptr, nullptr, 0, c.exec_of(body), c.st);
-    c.cond_begin(h, cudaGraphCondTypeIf, body);
-    cgs_dev(c, false);
-    ortho_decide2(state.p, d_proj, c.st);
-    c.cond_end();
-    ortho_final(state.p, d_proj, c.st);
-    ortho_store(state.p, W.p, MW.p, d_sol.p, d_mxx.p, nslots, N, c.d_err, c.st);
-    ortho_advance(state.p, recalc_period, nslots, c.st);
+    OrthoState* s = dev();
+    for (int sweep = 1; sweep <= 2; ++sweep) {  // the second one runs where the first asked for it
+      hist_dots(hs, d_mxx.p, &s->k, MW.p, N, d_hbeta, sweep == 1 ? d_proj + 1 : nullptr, c.st,
+                sweep == 2 ? &s->second : nullptr);
+      ortho_project(hs, d_sol.p, d_mxx.p, s, sweep, d_hbeta, W.p, MW.p, N, d_proj, err, c.st);
+    }
+    ortho_commit(hs, s, d_proj, W.p, MW.p, d_sol.p, d_mxx.p, slots, recalc_period, Res0, N, d_alpha, err,
+                 c.st);
   }
-  void minimize_dev(Ctx& c, T* X, const T* B, const T* Res0, T* Res, const TermParams& tp) {
-    const T* a[1] = {MW.p};
-    const T* b[1] = {Res0};
-    dots(c.red, 1, a, b, N, d_alpha, 0, c.st);
-    const T* sx[1] = {W.p};
-    axpys(1, d_alpha, nullptr, 1.0, sx, X, N, c.st);
-    spmv(*A, T(-1), X, T(1), B, Res, c.st, &state.p->recalc);
-    const T* mx[1] = {MW.p};
-    axpys(1, d_alpha, nullptr, -1.0, mx, Res, N, c.st, &state.p->update);
-    const T* r[1] = {Res};
-    dots(c.red, 1, r, r, N, d_rn, 1, c.st);
-    minimize_check(state.p, d_rn, tp, c.d_err, c.st);
+  void minimize_dev(Ctx& c, T* X, const T* B, T* Res, const TermParams& tp, int* err) {
+    ortho_minimize(hs, dev(), d_sol.p, d_mxx.p, d_alpha, X, Res, N, tp, err, c.st);
+    spmv(*A, T(-1), X, T(1), B, Res, c.st, &dev()->recalc);
+    ortho_check(hs, dev(), Res, N, tp, err, c.st);
+  }
+
+  // ---- host-driven form on the same kernels (histories up to kHistMax) ------------------------------------------
+  // One host round trip per correction: AddSol and MinimizeResidual run on the device's decisions, and the host reads
+  // the state afterwards.  A correction with nothing independent of the history left in it (stored as zero, the
+  // iterate and the residual unchanged) is then redone in the reference's order, with its re-orthonormalisation loop
+  // and random restarts.
+  int* ignored = nullptr;  // error word of the kernels' checks; the host makes them on the fetched values
+  void begin(Ctx& c, const TermParams& tp) {
+    alloc_dev(c);
+    if (!ignored) ignored = c.flag();
+    level_begin(dev(), d_norm, tp, c.st);
+    clear();
+  }
+  void restart(Ctx& c) {
+    iter_begin(dev(), cap, c.st);
+    clear();
+  }
+  // W holds a new correction; returns the new residual norm
+  double add_and_minimize(Ctx& c, T* X, const T* B, const T* Res0, T* Res, double rn_old, const TermParams& tp) {
+    add_sol_dev(c, Res0, cap + 1, ignored);
+    minimize_dev(c, X, B, Res, tp, ignored);
+    c.fetch(d_state, kStateScalars + 2);
+    const double* h = c.hscal + (d_state - c.dscal.p);
+    OrthoState s;
+    std::memcpy(&s, h, sizeof(s));
+    const double nM = std::sqrt(h[kStateScalars + 1]);
+    if (!std::isfinite(nM) || !std::isfinite(h[kStateScalars]))
+      throw Error(BSGPU_ERR_ARITHMETIC, "Orthonormalization: norm of matrix*solution is NaN/Inf");
+    if (!s.cancel) {
+      cancellation = false;
+      used_more_cycles = false;
+      ++k;
+      return checked_residual(s.rn, rn_old);
+    }
+    double rel = s.rel, scale = nM;
+    if (!(nM > 0)) {
+      random_restart(c, W.p, MW.p);
+      scale = c.hscal[d_norm - c.dscal.p];
+      rel = -1.0;
+    }
+    axpby(T(1.0 / scale), MW.p, T(0), MW.p, N, c.st);
+    axpby(T(1.0 / scale), W.p, T(0), W.p, N, c.st);
+    add_sol_tail(c, W.p, MW.p, rel);
+    copy_vec(Sol[k - 1].p, (const T*)W.p, N, c.st);
+    copy_vec(Mxx[k - 1].p, (const T*)MW.p, N, c.st);
+    return minimize(c, X, B, Res0, Res, rn_old);
   }
 };
 
@@ -1166,7 +1204,25 @@ struct OrthoMGT : Solver<T> {
     const double r0 = ortho.norm(c, Res0.p);
     double rn = r0;
     this->history.assign(1, r0);
-    ortho.clear();
+    const TermParams tp = term.params();
+    const bool dev = ortho.cap < kHistMax;  // a pre-smoother and a coarse correction may start from cap - 1 entries
+    if (dev)
+      ortho.begin(c, tp);
+    else
+      ortho.clear();
+    // one correction by `sv`: AddSol and MinimizeResidual; returns the new residual norm
+    auto correction = [&](Solver<T>* sv) {
+      if (dev) {
+        ortho.need_slots(c, ortho.k + 1);
+        if (!sv->overwrites()) fill(T(0), ortho.W.p, N, c.st);
+        sv->solve(c, ortho.W.p, Res.p, true);
+        return ortho.add_and_minimize(c, X, B, Res0.p, Res.p, rn, tp);
+      }
+      T* w = ortho.next_sol(c);
+      sv->solve(c, w, Res.p, true);
+      ortho.add_sol(c);
+      return ortho.minimize(c, X, B, Res0.p, Res.p, rn);
+    };
     this->converged = false;
     for (int iIter = 1;; ++iIter) {
       auto st = term(iIter, r0, rn);
@@ -1177,14 +1233,14 @@ struct OrthoMGT : Solver<T> {
       if (ortho.full() ) {
         // history capacity reached: restart the minimisation from the current iterate
         copy_vec(Res0.p, Res.p, N, c.st);
-        ortho.clear();
+        if (dev)
+          ortho.restart(c);
+        else
+          ortho.clear();
       }
       if (pre && (pre_on == nullptr || *pre_on)) {
         // pre-smoother (OrthonormalizationMultigrid.cs:893-915)
-        T* pc = ortho.next_sol(c);
-        pre->solve(c, pc, Res.p, true);
-        ortho.add_sol(c);
-        rn = ortho.minimize(c, X, B, Res0.p, Res.p, rn);
+        rn = correction(pre.get());
         st = term(iIter, r0, rn);
         if (!st.first) {
           this->converged = st.second;
@@ -1192,10 +1248,7 @@ struct OrthoMGT : Solver<T> {
         }
       }
       if (coarse) {
-        T* vl = ortho.next_sol(c);
-        coarse->solve(c, vl, Res.p, true);
-        ortho.add_sol(c);
-        rn = ortho.minimize(c, X, B, Res0.p, Res.p, rn);
+        rn = correction(coarse.get());
         st = term(iIter, r0, rn);
         if (!st.first) {
           this->converged = st.second;
@@ -1206,10 +1259,7 @@ struct OrthoMGT : Solver<T> {
       if (post) {
         for (int g = 0; g < sweeps; ++g) {
           if (ortho.full()) break;
-          T* pc = ortho.next_sol(c);
-          post->solve(c, pc, Res.p, true);
-          ortho.add_sol(c);
-          rn = ortho.minimize(c, X, B, Res0.p, Res.p, rn);
+          rn = correction(post.get());
           st = term(iIter, r0, rn);
           if (!st.first) {
             this->converged = st.second;
@@ -1247,10 +1297,11 @@ struct OrthoMGT : Solver<T> {
     if (pre) pre->prepare_graph(c);
   }
   void correction_dev(Ctx& c, Solver<T>* sv, T* X, const T* B, const TermParams& tp) {
-    T* w = ortho.next_sol_dev(c);
+    T* w = ortho.W.p;
+    if (!sv->overwrites()) fill(T(0), w, N, c.st);
     sv->solve_graph(c, w, Res.p, true);
-    ortho.add_sol_dev(c);
-    ortho.minimize_dev(c, X, B, Res0.p, Res.p, tp);
+    ortho.add_sol_dev(c, Res0.p, ortho.nslots, c.d_err);
+    ortho.minimize_dev(c, X, B, Res.p, tp, c.d_err);
   }
   // a correction recorded inside an IF node on (active && !cancel && k < cap) (post-smoother sweeps) or on
   // `active` alone
@@ -1968,7 +2019,7 @@ struct FlexGMRES : Solver<double>, RecordedSolve {
       dZ.alloc(m);
       BSGPU_CUDA(cudaMemcpy(dV.p, pv.data(), (m + 1) * sizeof(double*), cudaMemcpyHostToDevice));
       BSGPU_CUDA(cudaMemcpy(dZ.p, pz.data(), m * sizeof(double*), cudaMemcpyHostToDevice));
-      hsV.init(m + 1);
+      hsV.init(m + 1, c.st);
       fst.alloc(1);
       BSGPU_CUDA(cudaMemset(fst.p, 0, sizeof(FgState)));
       fa.m = m;
@@ -1988,6 +2039,7 @@ struct FlexGMRES : Solver<double>, RecordedSolve {
       d_rn = c.scal(1);
       BSGPU_CUDA(cudaMallocHost(&h_fst, sizeof(FgState)));
       BSGPU_CUDA(cudaMallocHost(&h_hist, fa.hcap * sizeof(double)));
+      BSGPU_CUDA(cudaStreamSynchronize(nullptr));  // the copies and fills above, before c.st uses them
     }
     c.graph_init();
     require(pc && pc->graphable() && (!pc2 || pc2->graphable()),
@@ -2565,6 +2617,7 @@ Tree* build_tree(const Matrix* A, const bsgpu_solver_config& cfg, const Operator
       throw Error(BSGPU_ERR_ARGUMENT, "unknown solver kind");
   }
   BSGPU_CUDA(cudaStreamSynchronize(t->ctx->st));
+  BSGPU_CUDA(cudaStreamSynchronize(nullptr));  // set-up copies on the legacy stream
   return t.release();
 }
 

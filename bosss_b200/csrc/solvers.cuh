@@ -114,6 +114,8 @@ struct Solver {
   // X: initial guess in, solution out (device); B: right-hand side (device).  zero_guess: X is known to be 0.
   virtual void solve(Ctx& c, T* X, const T* B, bool zero_guess) = 0;
   virtual int nested() const { return 0; }
+  // whether solve with zero_guess writes every entry of X without reading it (X need not hold zeros then)
+  virtual bool overwrites() const { return false; }
   // Graph capture (Ctx::capturing): whether solve_graph can be recorded into a CUDA graph, the buffers it needs
   // (allocated before the capture), and the recorded form of solve, whose decisions are taken on the device.
   // Solvers without host decisions record solve itself.
