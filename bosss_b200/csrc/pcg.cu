@@ -10,7 +10,6 @@ namespace bsgpu {
 
 namespace {
 
-constexpr int kThreads = 256;       // large systems
 constexpr int kThreadsOne = 512;    // one tile per CTA: fewer arrivals at the barrier
 
 // Vectors that other SMs write during the kernel are read from L2.
@@ -96,16 +95,16 @@ __device__ __forceinline__ Vec<ST, V> ldv_value(const ST* ptr, uint64_t pol) {
 
 // Block rows of a uniform matrix: SPLIT * NP threads per block row, thread (s, r) sums the blocks s, s + SPLIT, ...
 // of DOF row r; the partial sums meet in shared memory and the threads with s = 0 own the row.
-template <typename T, int NP, int V, int SPLIT, typename ST, int THREADS, int MINCTAS = 1>
+template <typename T, int NP, int V, int SPLIT, typename ST, int THREADS, int MINCTAS = 0>
 struct UniformRows {
   using Value = T;
   static constexpr int kV = V;
   static constexpr int kT = THREADS;
-  [[maybe_unused]] static constexpr int kMinCtas = MINCTAS;
+  [[maybe_unused]] static constexpr int kMinCtas = MINCTAS > 0 ? MINCTAS : 1;
   // blocks of 15 and 20 exchange the new residual through shared memory (24^3 p = 3 FP64: 74 us per iteration against
   // 79 with every thread recomputing its block's residual); smaller ones recompute it (64^3 p = 1: 71 against 89)
   [[maybe_unused]] static constexpr bool kExchange = NP >= 15;
-  static constexpr bool kCached = MINCTAS == 1;  // one tile per CTA
+  static constexpr bool kCached = MINCTAS == 0;  // one tile per CTA (small kernel)
   static constexpr int RT = NP * SPLIT;
   static constexpr int BPC = THREADS / RT;
   const int64_t* __restrict__ rp;
@@ -847,10 +846,11 @@ template <typename T, typename ST, class F>
 bool pick_large(const Matrix& A, F&& f) {
   if (pick_uniform<T, ST>(A, [&](auto np, auto v) {
         constexpr int NP = decltype(np)::value, V = decltype(v)::value;
-        // CTAs per SM: 4 (64 registers); blocks of 10 stream better from 5.  At 32^3 p = 2 FP64 (179 MB) 55 us per
-        // iteration against 60, at 200^2 p = 4 (blocks of 15, 359 MB) 142 against 130.
-        constexpr int MINCTAS = NP == 10 ? 5 : 4;
-        return f(Tag<UniformRows<T, NP, V, 1, ST, kThreads, MINCTAS>>{});
+        // Few and large CTAs: a barrier takes as long as its arrivals (32^3 p = 1 FP64 15.2 us per iteration with two CTAs
+        // of 512 threads per SM, 17.2 with four of 256).  64 registers per thread; blocks of 10 stream better with 48 and
+        // more threads.
+        constexpr int THREADS = NP == 10 ? 640 : 512;
+        return f(Tag<UniformRows<T, NP, V, 1, ST, THREADS, 2>>{});
       }))
     return true;
   if constexpr (sizeof(ST) != 2) {
