@@ -93,20 +93,25 @@ __global__ void restrict_kernel(const T* __restrict__ in, const int64_t* __restr
 template <typename T>
 struct Acc { using type = T; };
 
-// Uniform Np x Np blocks, Np known at compile time.  A CTA owns BPC = blockDim/NP whole block rows; thread t is DOF
-// row r = t % NP of block row t / NP.  MODE 0: y = alpha*A*x + beta*z.  MODE 1: fused block-Jacobi update
+// Uniform Np x Np blocks, Np known at compile time.  A CTA owns BPC = blockDim / (SPLIT*NP) whole block rows; thread t is
+// DOF row r of block row t / (SPLIT*NP), and with SPLIT > 1 the SPLIT threads of a DOF row take every SPLIT-th block and
+// meet in shared memory (small systems are bound by a row's chain of blocks, not by bandwidth).  MODE 0: y = alpha*A*x + beta*z.  MODE 1: fused block-Jacobi update
 // y = x + alpha * Dinv * (z - A*x) (z = b), the block row's residual exchanged through shared memory.
-template <typename T, int NP, int V, int MODE, typename S = T>
+template <typename T, int NP, int V, int MODE, typename S = T, int SPLIT = 1>
 __global__ void __launch_bounds__(256) spmv_uniform_kernel(
     const int64_t* __restrict__ rp, const int32_t* __restrict__ ci, const S* __restrict__ vals,
     const T* x, const T* __restrict__ z, T* y, T alpha, T beta, int64_t nb,
     const T* __restrict__ dinv, const int* __restrict__ active, const int32_t* __restrict__ row_list = nullptr) {
   static_assert(NP % V == 0, "chunk width must divide the block size");
+  static_assert(MODE != 2 || SPLIT == 1, "row lists take whole rows per thread");
   if (active != nullptr && *active == 0) return;
-  const int BPC = blockDim.x / NP;  // block rows per CTA (the launch shape the autotuner picks)
+  constexpr int RT = NP * SPLIT;
+  const int BPC = blockDim.x / RT;  // block rows per CTA (the launch shape the autotuner picks)
   const int t = threadIdx.x;
-  const int lb = t / NP;
-  const int r = t - lb * NP;
+  const int lb = t / RT;
+  const int u = t - lb * RT;
+  const int s = SPLIT > 1 ? u / NP : 0;
+  const int r = u - s * NP;
   // MODE 2 (block Gauss-Seidel half-sweep): the block rows come from `row_list` (one colour; nb is the list
   // length) and the update is in place (x == y): all reads of x precede the barrier, the write follows it, and
   // no block row of the list reads another row of the list.
@@ -118,9 +123,7 @@ __global__ void __launch_bounds__(256) spmv_uniform_kernel(
   const uint64_t pol = policy_evict_first();
   T acc0 = 0, acc1 = 0;
   if (valid) {
-    const int64_t k0 = rp[i], k1 = rp[i + 1];
-    for (int64_t k = k0; k < k1; ++k) {
-      const int64_t j = ci[k];
+    auto block = [&](int64_t k, int64_t j) {
       const S* vb = vals + k * (NP * NP) + r * V;
       const T* xb = x + j * NP;
 #pragma unroll
@@ -135,31 +138,67 @@ __global__ void __launch_bounds__(256) spmv_uniform_kernel(
             acc0 = fma(widen<T>(a.a[q]), xv.a[q], acc0);
         }
       }
+    };
+    const int64_t k0 = rp[i], k1 = rp[i + 1];
+    if constexpr (V == 1 && sizeof(T) == 8) {
+      // odd block sizes in FP64: the next block's column is fetched while a block is multiplied (333x251 p = 4, 784 MB:
+      // 124 us, 137 without; with two values per load the plain loop is the faster one: 24^3 p = 2 14.4 against 16.4)
+      int64_t k = k0 + s;
+      int32_t j = k < k1 ? ci[k] : 0;
+      while (k < k1) {
+        const int64_t kk = k, jj = j;
+        k += SPLIT;
+        if (k < k1) j = ci[k];
+        block(kk, jj);
+      }
+    } else {
+      for (int64_t k = k0 + s; k < k1; k += SPLIT) block(k, ci[k]);
     }
   }
-  const T acc = acc0 + acc1;
+  T acc = acc0 + acc1;
+  __shared__ T q[MODE == 0 && SPLIT == 1 ? 1 : 256];
+  if constexpr (SPLIT > 1) {
+    q[t] = acc;
+    __syncthreads();
+    if (s == 0) {
+#pragma unroll
+      for (int p = 1; p < SPLIT; ++p)
+        if (valid) acc += q[t + p * NP];
+    }
+  }
   const int64_t g = i * NP + r;
   if constexpr (MODE == 0) {
-    if (valid) {
+    if (valid && s == 0) {
       T out = alpha * acc;
       if (z != nullptr) out = fma(beta, z[g], out);
       y[g] = out;
     }
   } else {
-    __shared__ T q[256];
-    q[t] = valid ? (z[g] - acc) : T(0);
+    if constexpr (SPLIT > 1) __syncthreads();
+    if (s == 0) q[t] = valid ? (z[g] - acc) : T(0);
     __syncthreads();
+    T s0 = 0, s1 = 0;
     if (valid) {
       const T* D = dinv + i * (NP * NP) + r;
-      const T* qb = q + lb * NP;
-      T s0 = 0, s1 = 0;
+      const T* qb = q + lb * RT;
 #pragma unroll
-      for (int c = 0; c < NP; c += 2) {
-        s0 = fma(D[c * NP], qb[c], s0);
-        if (c + 1 < NP) s1 = fma(D[(c + 1) * NP], qb[c + 1], s1);
+      for (int c = 0; c < NP; c += 2 * SPLIT) {
+        if (c + s < NP) s0 = fma(D[(c + s) * NP], qb[c + s], s0);
+        if (c + SPLIT + s < NP) s1 = fma(D[(c + SPLIT + s) * NP], qb[c + SPLIT + s], s1);
       }
-      y[g] = fma(alpha, s0 + s1, x[g]);
     }
+    T d = s0 + s1;
+    if constexpr (SPLIT > 1) {
+      __syncthreads();
+      q[t] = d;
+      __syncthreads();
+      if (s == 0) {
+#pragma unroll
+        for (int p = 1; p < SPLIT; ++p)
+          if (valid) d += q[t + p * NP];
+      }
+    }
+    if (valid && s == 0) y[g] = fma(alpha, d, x[g]);
   }
 }
 
@@ -254,12 +293,10 @@ __device__ __forceinline__ void typed_rows(int BPC, int64_t b0, int64_t nrows, c
   const uint64_t pol = policy_evict_first();
   T acc0 = 0, acc1 = 0;
   if (valid) {
-    const int64_t k0 = rp[i], k1 = rp[i + 1];
-    for (int64_t k = k0; k < k1; ++k) {
-      const int64_t j = ci[k];
-      const int sj = len[j] / NP;
-      const T* vb = vals + boff[k] + r * V;
-      const T* xb = x + i0[j];
+    const int64_t k1 = rp[i + 1];
+    auto block = [&](int sj, int64_t voff, int64_t xoff) {
+      const T* vb = vals + voff + r * V;
+      const T* xb = x + xoff;
       for (int sp = 0; sp < sj; ++sp) {
 #pragma unroll
         for (int c = 0; c < NP / V; ++c) {
@@ -274,6 +311,37 @@ __device__ __forceinline__ void typed_rows(int BPC, int64_t b0, int64_t nrows, c
               acc0 = fma(a.a[q], xv.a[q], acc0);
           }
         }
+      }
+    };
+    if constexpr (sizeof(T) == 4) {
+      // Two steps ahead the next block's column, one step ahead what hangs on it, so that a block's chain of lookups
+      // (column, then length and offsets) is over when its turn comes: 40^3 p = 2 FP32 (190 MB) 60 us, 72 with the
+      // lookups in place; with FP64 blocks, twice as long each, the plain loop is the faster one (84 against 89 us).
+      int64_t k = rp[i];
+      int32_t j1 = k + 1 < k1 ? ci[k + 1] : 0;
+      int64_t vo = 0, xo = 0;
+      int ln = 0;
+      if (k < k1) {
+        const int32_t j0 = ci[k];
+        ln = len[j0];
+        xo = i0[j0];
+        vo = boff[k];
+      }
+      for (; k < k1; ++k) {
+        const int sj = ln / NP;
+        const int64_t v0 = vo, x0 = xo;
+        if (k + 1 < k1) {
+          ln = len[j1];
+          xo = i0[j1];
+          vo = boff[k + 1];
+          if (k + 2 < k1) j1 = ci[k + 2];
+        }
+        block(sj, v0, x0);
+      }
+    } else {
+      for (int64_t k = rp[i]; k < k1; ++k) {
+        const int64_t j = ci[k];
+        block(len[j] / NP, boff[k], i0[j]);
       }
     }
   }
@@ -319,6 +387,25 @@ __global__ void __launch_bounds__(256) spmv_typed_kernel(
   else
     typed_rows<T, NP, 2, V, MODE>(bpc2, ((int64_t)blockIdx.x - cta1) * bpc2, n2, rows + n1, rp, ci, len, i0, boff,
                                   vals, x, z, y, alpha, beta, dinv, doff);
+}
+
+// y = alpha * Dinv * b for uniform blocks of NP (column-major blocks): one thread per DOF row, the block row's NP columns
+// in flight together.  64^3 p = 2 FP32 (105 MB of blocks): 24.4 us, 31.1 with a runtime block size.
+template <typename T, int NP>
+__global__ void __launch_bounds__(256) blockdiag_uniform_kernel(const T* __restrict__ dinv, T alpha,
+                                                                const T* __restrict__ b, T* __restrict__ y, int64_t N,
+                                                                const int* __restrict__ active) {
+  if (active != nullptr && *active == 0) return;
+  const uint64_t pol = policy_evict_first();
+  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < N; g += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = g / NP;
+    const T* D = dinv + i * (NP * NP) + (g - i * NP);
+    const T* bb = b + i * NP;
+    T s = 0;
+#pragma unroll
+    for (int c = 0; c < NP; ++c) s = fma(ldv_stream<T, 1>(D + c * NP, pol).a[0], __ldg(bb + c), s);
+    y[g] = alpha * s;
+  }
 }
 
 // y = alpha * Dinv * b (block diagonal, column-major blocks)
@@ -450,6 +537,7 @@ std::vector<int64_t> rowmajor_offsets(const Matrix& M) {
 
 int conv_grid(int64_t nnzb) { return (int)std::min<int64_t>(std::max<int64_t>(nnzb, 1), 1 << 20); }
 
+// block sizes of the in-place row updates (and of the FP16 copies)
 bool specialised(const Matrix& A) {
   if (!A.uniform) return false;
   switch (A.Np) {
@@ -457,16 +545,33 @@ bool specialised(const Matrix& A) {
     default: return false;
   }
 }
+// block sizes with compile-time kernels for the product and the block-Jacobi update: the ones above and the odd sizes of
+// degree 1 to 4 in two and three dimensions (one value per load)
+bool unrolled(const Matrix& A) {
+  return specialised(A) || (A.uniform && A.V == 1 && (A.Np == 1 || A.Np == 3 || A.Np == 15 || A.Np == 35));
+}
+
+template <typename T, int NP, int V, int MODE, typename S = T, int SPLIT = 1>
+void launch_split(const Matrix& A, const S* vals, const T* x, const T* z, T* y, T alpha, T beta, const T* dinv,
+                  cudaStream_t st, const int* active) {
+  const int BPC = std::max(1, A.cta[MODE == 1 ? 1 : 0] / (NP * SPLIT));
+  const int64_t grid = (A.nb + BPC - 1) / BPC;
+  if (grid == 0) return;
+  spmv_uniform_kernel<T, NP, V, MODE, S, SPLIT><<<(unsigned)grid, BPC * NP * SPLIT, 0, st>>>(
+      A.rp.p, A.ci.p, vals, x, z, y, alpha, beta, A.nb, dinv, active);
+  BSGPU_CHECK_LAUNCH();
+}
 
 template <typename T, int NP, int V, int MODE, typename S = T>
 void launch_uniform(const Matrix& A, const S* vals, const T* x, const T* z, T* y, T alpha, T beta, const T* dinv,
                     cudaStream_t st, const int* active) {
-  const int BPC = std::max(1, A.cta[MODE == 1 ? 1 : 0] / NP);
-  const int64_t grid = (A.nb + BPC - 1) / BPC;
-  if (grid == 0) return;
-  spmv_uniform_kernel<T, NP, V, MODE, S><<<(unsigned)grid, BPC * NP, 0, st>>>(A.rp.p, A.ci.p, vals, x, z, y, alpha,
-                                                                             beta, A.nb, dinv, active);
-  BSGPU_CHECK_LAUNCH();
+  if constexpr (NP <= 20) {
+    // Up to here one thread per DOF row leaves most of the chip idle, and the row's chain of blocks is what takes the
+    // time: 64^2 p = 2 FP32 (24,576 rows) 4.4 us with four threads per row, 6.2 with one; 24^3 p = 2 (138,240 rows) 20.3
+    // against 16.4 us.
+    if (A.N <= 49152) return launch_split<T, NP, V, MODE, S, 4>(A, vals, x, z, y, alpha, beta, dinv, st, active);
+  }
+  launch_split<T, NP, V, MODE, S, 1>(A, vals, x, z, y, alpha, beta, dinv, st, active);
 }
 
 // FP16 values, FP32 vectors and arithmetic (the preconditioner's level matrices stored in half precision); uniform
@@ -533,9 +638,13 @@ template <typename T, int MODE>
 void dispatch(const Matrix& A, const T* vals, const T* x, const T* z, T* y, T alpha, T beta, const T* dinv,
               const int64_t* doff, cudaStream_t st, const int* active) {
   if (dispatch_typed<T, MODE>(A, vals, x, z, y, alpha, beta, dinv, doff, st, active)) return;
-  if (specialised(A)) {
+  if (unrolled(A)) {
     constexpr int VW = sizeof(T) == 8 ? 2 : 4;
     switch (A.Np) {
+      case 1: return launch_uniform<T, 1, 1, MODE>(A, vals, x, z, y, alpha, beta, dinv, st, active);
+      case 3: return launch_uniform<T, 3, 1, MODE>(A, vals, x, z, y, alpha, beta, dinv, st, active);
+      case 15: return launch_uniform<T, 15, 1, MODE>(A, vals, x, z, y, alpha, beta, dinv, st, active);
+      case 35: return launch_uniform<T, 35, 1, MODE>(A, vals, x, z, y, alpha, beta, dinv, st, active);
       case 20: return launch_uniform<T, 20, VW, MODE>(A, vals, x, z, y, alpha, beta, dinv, st, active);
       case 4: return launch_uniform<T, 4, VW, MODE>(A, vals, x, z, y, alpha, beta, dinv, st, active);
       case 10: return launch_uniform<T, 10, 2, MODE>(A, vals, x, z, y, alpha, beta, dinv, st, active);
@@ -832,6 +941,18 @@ namespace {
 template <typename T>
 void blockdiag_impl(const Matrix& A, const T* dinv, T alpha, const T* b, T* y, cudaStream_t st, const int* active) {
   if (A.N == 0) return;
+  if (A.uniform) {
+    const int g = (int)std::min<int64_t>((A.N + 255) / 256, (int64_t)num_sms() * 32);
+#define BSGPU_BD(NP)                                                              \
+  case NP:                                                                        \
+    blockdiag_uniform_kernel<T, NP><<<g, 256, 0, st>>>(dinv, alpha, b, y, A.N, active); \
+    BSGPU_CHECK_LAUNCH();                                                         \
+    return;
+    switch (A.Np) {
+      BSGPU_BD(1) BSGPU_BD(3) BSGPU_BD(4) BSGPU_BD(6) BSGPU_BD(10) BSGPU_BD(15) BSGPU_BD(20)
+    }
+#undef BSGPU_BD
+  }
   const int grid = (int)std::min<int64_t>((A.N + 255) / 256, (int64_t)num_sms() * 16);
   blockdiag_kernel<T><<<grid, 256, 0, st>>>(A.len.p, A.i0.p, A.row2blk.p, A.doff.p, dinv, alpha, b, y, A.N,
                                             A.uniform ? A.Np : 0, active);
@@ -892,7 +1013,7 @@ float time_launches(const Matrix& A, int mode, const T* dinv, const T* x, const 
 
 template <typename T>
 void autotune_impl(const Matrix& A, int mode, const T* dinv, cudaStream_t st) {
-  const bool tunable = A.typed || specialised(A) || A.half;
+  const bool tunable = A.typed || unrolled(A) || A.half;
   if (!tunable || A.tuned[mode] || A.N == 0) return;
   int dev = 0;
   BSGPU_CUDA(cudaGetDevice(&dev));
