@@ -32,6 +32,23 @@ def _is_device(a) -> bool:
     return hasattr(a, "is_cuda") and a.is_cuda
 
 
+_raw_stream = None
+
+
+def _current_stream() -> int:
+    """torch's current stream on the current device.  torch.cuda.current_stream() builds a Stream object per call,
+    3.5 us of the 8.2 us that a small product took; torch's own accessor of the raw handle is used where it exists."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        get, dev = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+        if get is not None and dev is not None:
+            _raw_stream = lambda: get(dev())  # noqa: E731
+        else:
+            _raw_stream = lambda: torch.cuda.current_stream().cuda_stream  # noqa: E731
+    return _raw_stream()
+
+
 class BlockMsrMatrix:
     """Device-resident block-sparse matrix with dense Np x Np (or nspc*Np) blocks."""
 
@@ -135,10 +152,8 @@ class BlockMsrMatrix:
                                                              nat.ptr(acc), None))
             return acc
         if _is_device(a):
-            import torch
-            stream = torch.cuda.current_stream().cuda_stream
             nat.check(nat.lib().bsgpu_matrix_spmv_device(self._h, float(alpha), nat.ptr(a), float(beta), nat.ptr(acc),
-                                                         C.c_void_p(stream)))
+                                                         _current_stream()))
         else:
             if acc.dtype != np.float64 or not acc.flags.c_contiguous:
                 raise ValueError("acc must be a contiguous float64 array")
