@@ -1114,8 +1114,10 @@ struct OrthoT {
     ortho_commit(hs, s, d_proj, W.p, MW.p, d_sol.p, d_mxx.p, slots, recalc_period, Res0, N, d_alpha, err,
                  c.st);
   }
-  void minimize_dev(Ctx& c, T* X, const T* B, T* Res, const TermParams& tp, int* err) {
+  // recompute: whether the residual can need the product (with the host's k it is known unless the correction cancels)
+  void minimize_dev(Ctx& c, T* X, const T* B, T* Res, const TermParams& tp, int* err, bool recompute = true) {
     ortho_minimize(hs, dev(), d_sol.p, d_mxx.p, d_alpha, X, Res, N, tp, err, c.st);
+    if (!recompute) return;
     spmv(*A, T(-1), X, T(1), B, Res, c.st, &dev()->recalc);
     ortho_check(hs, dev(), Res, N, tp, err, c.st);
   }
@@ -1139,7 +1141,7 @@ struct OrthoT {
   // W holds a new correction; returns the new residual norm
   double add_and_minimize(Ctx& c, T* X, const T* B, const T* Res0, T* Res, double rn_old, const TermParams& tp) {
     add_sol_dev(c, Res0, cap + 1, ignored);
-    minimize_dev(c, X, B, Res, tp, ignored);
+    minimize_dev(c, X, B, Res, tp, ignored, recalc_period <= 1 || (k + 1) % recalc_period == 0);
     c.fetch(d_state, kStateScalars + 2);
     const double* h = c.hscal + (d_state - c.dscal.p);
     OrthoState s;
