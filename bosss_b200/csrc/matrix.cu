@@ -273,8 +273,9 @@ __global__ void __launch_bounds__(256) spmv_general_kernel(
 // listed in `rows`; a CTA owns blockDim / (NS*NP) of them, thread t being DOF row r of list entry t / (NS*NP), as in
 // the uniform kernel, so the row length is a compile-time constant.  A block in column j has len[j] / NP species
 // sub-blocks of NP columns, each streamed with the fully unrolled chunk loop of the uniform kernel (V divides NP,
-// so no chunk straddles a species boundary and there is no scalar tail).
-template <typename T, int NP, int NS, int V, int MODE>
+// so no chunk straddles a species boundary and there is no scalar tail).  SPLIT threads share a row, each with every
+// SPLIT-th block (small systems, see launch_typed): their sums meet in shared memory.
+template <typename T, int NP, int NS, int V, int MODE, int SPLIT>
 __device__ __forceinline__ void typed_rows(int BPC, int64_t b0, int64_t nrows, const int32_t* __restrict__ rows,
                                            const int64_t* __restrict__ rp, const int32_t* __restrict__ ci,
                                            const int32_t* __restrict__ len, const int64_t* __restrict__ i0,
@@ -283,10 +284,13 @@ __device__ __forceinline__ void typed_rows(int BPC, int64_t b0, int64_t nrows, c
                                            T alpha, T beta, const T* __restrict__ dinv,
                                            const int64_t* __restrict__ doff) {
   constexpr int I = NP * NS;
+  constexpr int RT = I * SPLIT;
   static_assert(NP % V == 0, "chunk width must divide the species block");
   const int t = threadIdx.x;
-  const int lb = t / I;
-  const int r = t - lb * I;
+  const int lb = t / RT;
+  const int u = t - lb * RT;
+  const int s = SPLIT > 1 ? u / I : 0;
+  const int r = u - s * I;
   const int64_t b = b0 + lb;
   const bool valid = (lb < BPC) && (b < nrows);
   const int64_t i = valid ? rows[b] : 0;
@@ -317,8 +321,8 @@ __device__ __forceinline__ void typed_rows(int BPC, int64_t b0, int64_t nrows, c
       // Two steps ahead the next block's column, one step ahead what hangs on it, so that a block's chain of lookups
       // (column, then length and offsets) is over when its turn comes: 40^3 p = 2 FP32 (190 MB) 60 us, 72 with the
       // lookups in place; with FP64 blocks, twice as long each, the plain loop is the faster one (84 against 89 us).
-      int64_t k = rp[i];
-      int32_t j1 = k + 1 < k1 ? ci[k + 1] : 0;
+      int64_t k = rp[i] + s;
+      int32_t j1 = k + SPLIT < k1 ? ci[k + SPLIT] : 0;
       int64_t vo = 0, xo = 0;
       int ln = 0;
       if (k < k1) {
@@ -327,52 +331,71 @@ __device__ __forceinline__ void typed_rows(int BPC, int64_t b0, int64_t nrows, c
         xo = i0[j0];
         vo = boff[k];
       }
-      for (; k < k1; ++k) {
+      for (; k < k1; k += SPLIT) {
         const int sj = ln / NP;
         const int64_t v0 = vo, x0 = xo;
-        if (k + 1 < k1) {
+        if (k + SPLIT < k1) {
           ln = len[j1];
           xo = i0[j1];
-          vo = boff[k + 1];
-          if (k + 2 < k1) j1 = ci[k + 2];
+          vo = boff[k + SPLIT];
+          if (k + 2 * SPLIT < k1) j1 = ci[k + 2 * SPLIT];
         }
         block(sj, v0, x0);
       }
     } else {
-      for (int64_t k = rp[i]; k < k1; ++k) {
+      for (int64_t k = rp[i] + s; k < k1; k += SPLIT) {
         const int64_t j = ci[k];
         block(len[j] / NP, boff[k], i0[j]);
       }
     }
   }
-  const T acc = acc0 + acc1;
+  T acc = acc0 + acc1;
+  __shared__ T q[MODE == 0 && SPLIT == 1 ? 1 : 256];
+  if constexpr (SPLIT > 1) {
+    q[t] = acc;
+    __syncthreads();
+    if (valid && s == 0) {
+#pragma unroll
+      for (int p = 1; p < SPLIT; ++p) acc += q[t + p * I];
+    }
+  }
   const int64_t g = valid ? i0[i] + r : 0;
   if constexpr (MODE == 0) {
-    if (valid) {
+    if (valid && s == 0) {
       T out = alpha * acc;
       if (z != nullptr) out = fma(beta, z[g], out);
       y[g] = out;
     }
   } else {
-    __shared__ T q[256];
-    q[t] = valid ? (z[g] - acc) : T(0);
+    if constexpr (SPLIT > 1) __syncthreads();
+    if (s == 0) q[t] = valid ? (z[g] - acc) : T(0);
     __syncthreads();
+    T s0 = 0, s1 = 0;
     if (valid) {
       const T* D = dinv + doff[i] + r;
-      const T* qb = q + lb * I;
-      T s0 = 0, s1 = 0;
+      const T* qb = q + lb * RT;
 #pragma unroll
-      for (int c = 0; c < I; c += 2) {
-        s0 = fma(D[c * I], qb[c], s0);
-        if (c + 1 < I) s1 = fma(D[(c + 1) * I], qb[c + 1], s1);
+      for (int c = 0; c < I; c += 2 * SPLIT) {
+        if (c + s < I) s0 = fma(D[(c + s) * I], qb[c + s], s0);
+        if (c + SPLIT + s < I) s1 = fma(D[(c + SPLIT + s) * I], qb[c + SPLIT + s], s1);
       }
-      y[g] = fma(alpha, s0 + s1, x[g]);
     }
+    T d = s0 + s1;
+    if constexpr (SPLIT > 1) {
+      __syncthreads();
+      q[t] = d;
+      __syncthreads();
+      if (valid && s == 0) {
+#pragma unroll
+        for (int p = 1; p < SPLIT; ++p) d += q[t + p * I];
+      }
+    }
+    if (valid && s == 0) y[g] = fma(alpha, d, x[g]);
   }
 }
 
 // One launch for both species counts: CTAs [0, cta1) take the one-species rows, the rest the two-species rows.
-template <typename T, int NP, int V, int MODE>
+template <typename T, int NP, int V, int MODE, int SPLIT>
 __global__ void __launch_bounds__(256) spmv_typed_kernel(
     const int64_t* __restrict__ rp, const int32_t* __restrict__ ci, const int32_t* __restrict__ len,
     const int64_t* __restrict__ i0, const int64_t* __restrict__ boff, const int32_t* __restrict__ rows,
@@ -380,13 +403,13 @@ __global__ void __launch_bounds__(256) spmv_typed_kernel(
     const T* __restrict__ z, T* __restrict__ y, T alpha, T beta, const T* __restrict__ dinv,
     const int64_t* __restrict__ doff, const int* __restrict__ active) {
   if (active != nullptr && *active == 0) return;
-  const int bpc1 = blockDim.x / NP, bpc2 = blockDim.x / (2 * NP);
+  const int bpc1 = blockDim.x / (NP * SPLIT), bpc2 = blockDim.x / (2 * NP * SPLIT);
   if ((int64_t)blockIdx.x < cta1)
-    typed_rows<T, NP, 1, V, MODE>(bpc1, (int64_t)blockIdx.x * bpc1, n1, rows, rp, ci, len, i0, boff, vals, x, z, y,
-                                  alpha, beta, dinv, doff);
+    typed_rows<T, NP, 1, V, MODE, SPLIT>(bpc1, (int64_t)blockIdx.x * bpc1, n1, rows, rp, ci, len, i0, boff, vals, x, z,
+                                         y, alpha, beta, dinv, doff);
   else
-    typed_rows<T, NP, 2, V, MODE>(bpc2, ((int64_t)blockIdx.x - cta1) * bpc2, n2, rows + n1, rp, ci, len, i0, boff,
-                                  vals, x, z, y, alpha, beta, dinv, doff);
+    typed_rows<T, NP, 2, V, MODE, SPLIT>(bpc2, ((int64_t)blockIdx.x - cta1) * bpc2, n2, rows + n1, rp, ci, len, i0,
+                                         boff, vals, x, z, y, alpha, beta, dinv, doff);
 }
 
 // y = alpha * Dinv * b for uniform blocks of NP (column-major blocks): one thread per DOF row, the block row's NP columns
@@ -599,17 +622,29 @@ void launch_general(const Matrix& A, const T* vals, const T* x, const T* z, T* y
   BSGPU_CHECK_LAUNCH();
 }
 
-template <typename T, int NP, int V, int MODE>
-void launch_typed(const Matrix& A, const T* vals, const T* x, const T* z, T* y, T alpha, T beta, const T* dinv,
-                  const int64_t* doff, cudaStream_t st, const int* active) {
-  const int threads = std::max(A.cta[MODE == 1 ? 1 : 0], 2 * NP);
-  const int64_t bpc1 = threads / NP, bpc2 = threads / (2 * NP);
+template <typename T, int NP, int V, int MODE, int SPLIT>
+void launch_typed_split(const Matrix& A, const T* vals, const T* x, const T* z, T* y, T alpha, T beta, const T* dinv,
+                        const int64_t* doff, cudaStream_t st, const int* active) {
+  const int threads = std::max(A.cta[MODE == 1 ? 1 : 0], 2 * NP * SPLIT);
+  const int64_t bpc1 = threads / (NP * SPLIT), bpc2 = threads / (2 * NP * SPLIT);
   const int64_t cta1 = (A.grp_n1 + bpc1 - 1) / bpc1, cta2 = (A.grp_n2 + bpc2 - 1) / bpc2;
   if (cta1 + cta2 == 0) return;
-  spmv_typed_kernel<T, NP, V, MODE><<<(unsigned)(cta1 + cta2), threads, 0, st>>>(
+  spmv_typed_kernel<T, NP, V, MODE, SPLIT><<<(unsigned)(cta1 + cta2), threads, 0, st>>>(
       A.rp.p, A.ci.p, A.len.p, A.i0.p, A.boff.p, A.grp_rows.p, A.grp_n1, A.grp_n2, cta1, vals, x, z, y, alpha, beta,
       dinv, doff, active);
   BSGPU_CHECK_LAUNCH();
+}
+
+template <typename T, int NP, int V, int MODE>
+void launch_typed(const Matrix& A, const T* vals, const T* x, const T* z, T* y, T alpha, T beta, const T* dinv,
+                  const int64_t* doff, cudaStream_t st, const int* active) {
+  // The limit of the uniform kernel (blocks of two species beside those of one, FP64, four threads per row against
+  // one): 24^3 p = 0 (13,824 rows) 5.8 against 9.2 us, 20^3 p = 1 6.2 against 11.3, 12^3 p = 3 14.4 against 32.8;
+  // past it 18^3 p = 2 (58,000) 16.4 against 20.5 but 100^2 p = 2 (60,000) 12.3 against 11.3 and 40^3 p = 2 104
+  // against 84.  FP32 turns at the same sizes.
+  if (A.N <= 49152)
+    return launch_typed_split<T, NP, V, MODE, 4>(A, vals, x, z, y, alpha, beta, dinv, doff, st, active);
+  launch_typed_split<T, NP, V, MODE, 1>(A, vals, x, z, y, alpha, beta, dinv, doff, st, active);
 }
 
 // the (Np, V) pairs of the typed kernels; false: not covered (the general kernel serves the matrix)

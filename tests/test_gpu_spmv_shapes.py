@@ -57,10 +57,13 @@ def test_product(cuda, Np, nb, two):
         assert np.all(np.abs(yd.double().cpu().numpy() - 1.5 * (A @ x)) <= n * eps * size)
 
 
-@pytest.mark.parametrize("Np,nb", [(1, 130), (3, 16384), (3, 16385), (6, 100), (15, 60), (15, 3277), (20, 2458), (35, 40)])
-def test_block_jacobi(cuda, Np, nb):
+@pytest.mark.parametrize("Np,nb,two", [
+    (1, 130, False), (3, 16384, False), (3, 16385, False), (6, 100, False), (15, 60, False), (15, 3277, False),
+    (20, 2458, False), (35, 40, False), (1, 1, True), (1, 300, True), (4, 37, True), (10, 1000, True), (20, 500, True),
+    (20, 3000, True)])
+def test_block_jacobi(cuda, Np, nb, two):
     from bosss_b200.solvers import BlockJacobiConfig, BlockMsrMatrix, MultigridOperator
-    rp, ci, values, nspc, A, i0 = _system(Np, nb, False, Np + nb)
+    rp, ci, values, nspc, A, i0 = _system(Np, nb, two, Np + nb)
     op = MultigridOperator(BlockMsrMatrix.from_bsr(Np, rp, ci, values, nspc), MultigridOperator.Eye)
     D = sp.block_diag([sp.csr_matrix(np.linalg.inv(A[a:b, a:b].toarray())) for a, b in zip(i0, i0[1:])], format="csr")
     rng = np.random.default_rng(9)
