@@ -92,7 +92,7 @@ void level_begin(OrthoState* s, const double* r0_in, TermParams tp, cudaStream_t
 void iter_begin(OrthoState* s, int cap, cudaStream_t st);
 // end of an iteration: iterations += active, iter += 1, active = active && term(iter, r0, rn)
 void iter_end(OrthoState* s, TermParams tp, cudaStream_t st);
-// y -= sum_{j<*k} beta[j] x[j]; one launch (the single-vector form of hist_axpy2)
+// y -= sum_{j<*k} beta[j] x[j]; one launch
 void hist_axpy1(const double* const* x, const int* k, int kmax, const double* beta, double* y, int64_t n,
                 cudaStream_t st);
 

@@ -93,9 +93,10 @@ __global__ void restrict_kernel(const T* __restrict__ in, const int64_t* __restr
 template <typename T>
 struct Acc { using type = T; };
 
-// Uniform Np x Np blocks, Np known at compile time.  A CTA owns BPC = blockDim / (SPLIT*NP) whole block rows; thread t is
-// DOF row r of block row t / (SPLIT*NP), and with SPLIT > 1 the SPLIT threads of a DOF row take every SPLIT-th block and
-// meet in shared memory (small systems are bound by a row's chain of blocks, not by bandwidth).  MODE 0: y = alpha*A*x + beta*z.  MODE 1: fused block-Jacobi update
+// Uniform Np x Np blocks, Np known at compile time.  A CTA owns BPC = blockDim / (SPLIT*NP) whole block rows; thread t
+// is DOF row r of block row t / (SPLIT*NP), and with SPLIT > 1 the SPLIT threads of a DOF row take every SPLIT-th block
+// and meet in shared memory (small systems are bound by a row's chain of blocks, not by bandwidth).
+// MODE 0: y = alpha*A*x + beta*z.  MODE 1: fused block-Jacobi update
 // y = x + alpha * Dinv * (z - A*x) (z = b), the block row's residual exchanged through shared memory.
 template <typename T, int NP, int V, int MODE, typename S = T, int SPLIT = 1>
 __global__ void __launch_bounds__(256) spmv_uniform_kernel(

@@ -37,6 +37,7 @@ __device__ __forceinline__ Vec<T, V> ldv_cg(const T* ptr) {
 // A vector in plain memory.
 template <typename T, int V>
 struct PlainVec {
+  static constexpr bool kSlots = false;
   const T* x;
   template <int NV>
   __device__ __forceinline__ void load(int64_t idx, Vec<T, V> (&out)[NV]) const {
@@ -45,9 +46,37 @@ struct PlainVec {
   }
 };
 
+// The operand's blocks gathered in shared memory, one slot per block of a block row.
+template <typename T, int V>
+struct SlotVec {
+  static constexpr bool kSlots = true;
+  const T* x;
+  template <int NV>
+  __device__ __forceinline__ void load(int64_t idx, Vec<T, V> (&out)[NV]) const {
+#pragma unroll
+    for (int c = 0; c < NV; ++c) {
+      if constexpr (sizeof(T) == 8 && V == 2) {
+        const double2 v = *reinterpret_cast<const double2*>(x + idx + c * V);
+        out[c].a[0] = v.x;
+        out[c].a[1] = v.y;
+      } else if constexpr (sizeof(T) == 4 && V == 4) {
+        const float4 v = *reinterpret_cast<const float4*>(x + idx + c * V);
+        out[c].a[0] = v.x;
+        out[c].a[1] = v.y;
+        out[c].a[2] = v.z;
+        out[c].a[3] = v.w;
+      } else {
+#pragma unroll
+        for (int u = 0; u < V; ++u) out[c].a[u] = x[idx + c * V + u];
+      }
+    }
+  }
+};
+
 // A vector of packets at epoch `ep`.
 template <typename T, int V>
 struct PacketVec {
+  static constexpr bool kSlots = false;
   const uint64_t* w;
   unsigned ep;
   unsigned int* fail;
@@ -92,6 +121,9 @@ __device__ __forceinline__ Vec<ST, V> ldv_value(const ST* ptr, uint64_t pol) {
   else
     return ldv_stream<ST, V>(ptr, pol);
 }
+
+// blocks per block row up to which the operand is gathered once per CTA
+constexpr int kRowBlocks = 8;
 
 // Block rows of a uniform matrix: SPLIT * NP threads per block row, thread (s, r) sums the blocks s, s + SPLIT, ...
 // of DOF row r; the partial sums meet in shared memory and the threads with s = 0 own the row.
@@ -158,6 +190,13 @@ struct UniformRows {
     own = valid && s == 0;
     g = i * NP + r;
   }
+  // where the operand of the row's block number k is kept by the kernel that gathers it (kRowBlocks blocks per row)
+  static constexpr int kSplit = SPLIT, kNP = NP;
+  // Gathering pays while a thread keeps few elements (kRowBlocks / SPLIT), us per iteration with and without, FP64:
+  // split 4: 16^3 p = 1 6.9 / 8.0, 11^3 p = 2 8.6 / 10.2, 9^3 p = 3 9.4 / 10.4; split 2: 64^2 p = 2 6.6 / 7.3,
+  // 14^3 p = 2 9.0 / 9.9, but 12^3 p = 3 16.9 / 14.2; split 1 (spills): 26^3 p = 1 12.8 / 10.1, 100^2 p = 2 14.0 / 10.9
+  static constexpr bool kGathers = kCached && (SPLIT == 4 || (SPLIT == 2 && NP <= 10));
+  __device__ __forceinline__ int slot(int k) const { return (lb * kRowBlocks + k) * NP; }
   // the operand is loaded in groups of NV chunks (with packets a group is one wait)
   static constexpr int NC = NP / V;
   static constexpr int kGroup = !kCached ? 1 : (sizeof(T) == 8 ? 6 : 12) / V;
@@ -184,9 +223,13 @@ struct UniformRows {
   __device__ __forceinline__ T product(const Vector& x, T* sm) {
     T acc0 = 0, acc1 = 0;
     if (valid) {
-      const int64_t k1 = __ldg(rp + i + 1);
-      for (int64_t k = __ldg(rp + i) + s; k < k1; k += SPLIT) {
-        const int64_t x0 = (int64_t)__ldg(ci + k) * NP;
+      const int64_t k0 = __ldg(rp + i), k1 = __ldg(rp + i + 1);
+      for (int64_t k = k0 + s; k < k1; k += SPLIT) {
+        int64_t x0;
+        if constexpr (Vector::kSlots)
+          x0 = (int64_t)slot((int)(k - k0));
+        else
+          x0 = (int64_t)__ldg(ci + k) * NP;
         const ST* vb = vals + k * (NP * NP) + r * V;
 #pragma unroll
         for (int h = 0; h + NV <= NC; h += NV) group<NV>(x, vb, x0, h, acc0, acc1);
@@ -242,6 +285,7 @@ struct GeneralRows {
   static constexpr int kT = kRows * SPLIT;
   static constexpr int kMinCtas = ONE ? 1 : 4;
   static constexpr bool kExchange = false;
+  static constexpr bool kGathers = false;
   const int64_t* __restrict__ rp;
   const int32_t* __restrict__ ci;
   const int32_t* __restrict__ len;
@@ -409,10 +453,16 @@ __device__ __forceinline__ void grid_sums(double (&out)[K], const double* __rest
 }
 
 // The same sums exchanged as packets (w: K values per CTA): no counter and no fence, the arrival of a CTA's packet is
-// its arrival at the reduction.  Warp 0 collects, four packets per lane in flight.
-template <int K, int THREADS>
+// its arrival at the reduction.  Warp 0 collects, four packets per lane in flight.  `side` is a wait for other packets
+// that all warps finish in the meantime; warp 0 polls it along with the sums.
+struct NoSide {
+  __device__ __forceinline__ void poll() {}
+  __device__ __forceinline__ void finish() {}
+};
+
+template <int K, int THREADS, class Side>
 __device__ __forceinline__ bool exchange_sums(const double (&acc)[K], double (&out)[K], uint64_t* w, unsigned ep,
-                                              unsigned int* fail, double (*red)[2]) {
+                                              unsigned int* fail, double (*red)[2], Side&& side) {
   __shared__ double tot[2];
   __shared__ int failed;
   double v[K];
@@ -435,6 +485,7 @@ __device__ __forceinline__ bool exchange_sums(const double (&acc)[K], double (&o
       bool ready;
       do {
         ready = true;
+        side.poll();
 #pragma unroll
         for (int u = 0; u < 4; ++u)
           if (b0 + 32 * u < G) {
@@ -465,10 +516,17 @@ __device__ __forceinline__ bool exchange_sums(const double (&acc)[K], double (&o
     }
     if (lane == 0) failed = over;
   }
+  side.finish();
   sync_threads<THREADS>();
 #pragma unroll
   for (int k = 0; k < K; ++k) out[k] = tot[k];
   return failed == 0;
+}
+
+template <int K, int THREADS>
+__device__ __forceinline__ bool exchange_sums(const double (&acc)[K], double (&out)[K], uint64_t* w, unsigned ep,
+                                              unsigned int* fail, double (*red)[2]) {
+  return exchange_sums<K, THREADS>(acc, out, w, ep, fail, red, NoSide{});
 }
 
 // Grid barrier (all CTAs are resident: cooperative launch).  False when the bounded wait ran out somewhere.
@@ -561,8 +619,8 @@ struct CgScalars {
 // iteration.  With small blocks the vector phase recomputes the new residual of a whole block in each of the block's
 // threads (from the old one, two residual buffers) instead of exchanging it, and the scalars sit in shared memory, so
 // that no phase has a CTA barrier inside and the registers allow the occupancy that the stream of blocks needs.
-// Bound by HBM (or L2) traffic: 32^3 p = 1 FP64 (29 MB) 17 us per iteration (25 as four launches), 64^3 p = 1 (232 MB)
-// 71 us (74), 400^2 p = 1 (57 MB) 35 us (64).
+// Bound by HBM (or L2) traffic: 32^3 p = 1 FP64 (29 MB) 15 us per iteration (25 as four launches), 64^3 p = 1 (232 MB)
+// 69 us (74), 400^2 p = 1 (57 MB) 33 us (64).
 template <class Rows>
 __global__ void __launch_bounds__(Rows::kT, Rows::kMinCtas)
     pcg_kernel(Rows rows, PcgCall<typename Rows::Value> a, typename Rows::Value* __restrict__ r2,
@@ -688,11 +746,29 @@ __global__ void __launch_bounds__(Rows::kT, Rows::kMinCtas)
   c.end(a, ok);
 }
 
+// The end of a one-tile kernel: the last CTA leaves the epoch for the next launch.  A wait that ran out anywhere is an
+// error (the warp that gave up says so before its CTA's next sum).
+template <typename T>
+__device__ __forceinline__ void small_end(const PcgCall<T>& a, CgScalars& c, bool ok, unsigned ep,
+                                          unsigned int* __restrict__ state) {
+  if (threadIdx.x == 0) {
+    unsigned int failed;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(failed) : "l"(state + 1) : "memory");
+    ok = ok && failed == 0u;
+    if (atomicAdd(state + 2, 1u) == gridDim.x - 1) {
+      state[0] = ok ? ep : ep + 8;  // beyond every epoch that a CTA can have reached
+      state[1] = state[2] = 0u;
+      __threadfence();
+    }
+  }
+  c.end(a, ok);
+}
+
 // One tile per CTA: the rows' x, r, z, p and q stay in registers and the CTA's blocks in L1 for the whole solve.  What
 // other CTAs need - the direction p and the partial sums - goes through packets, so an iteration waits three times
 // for one store to be seen (p by its neighbours' products, p.q, and r.z with r.r) and never for a counter.
-// Bound by the latency of those exchanges: 64^2 p = 2 FP64 (24,576 unknowns) 7.4 us per iteration, 21 as four launches
-// of a graph; 24^3 p = 0 7.7 us (32 as nine launches).
+// Bound by the latency of those exchanges: 100^2 p = 2 FP64 (60,000 unknowns) 10.9 us per iteration, 40^3 p = 0 10.5;
+// 64^2 p = 2 7.3 us (21 as four launches of a graph).
 // No packet is overwritten before everybody has read it: the p of the next epoch is stored after the exchange of
 // r.z, which every CTA enters after its product; a sum of the next epoch after an exchange that every CTA enters
 // after having read the sum before.
@@ -782,12 +858,175 @@ __global__ void __launch_bounds__(Rows::kT) pcg_small_kernel(Rows rows, PcgCall<
       a.p[rows.g] = vp;
     }
   }
-  if (threadIdx.x == 0 && atomicAdd(state + 2, 1u) == gridDim.x - 1) {
-    state[0] = ok ? ep : ep + 8;  // beyond every epoch that a CTA can have reached
-    state[1] = state[2] = 0u;
-    __threadfence();
+  small_end(a, c, ok, ep, state);
+}
+
+// One value per block of a thread's share of its block row: element r of the block's operand, as packets of `z` (col:
+// its index, negative for none).
+template <typename T, int MB>
+struct Gather {
+  static constexpr int W = sizeof(T) / 4;
+  const uint64_t* __restrict__ z;
+  unsigned int* fail;
+  int col[MB];
+  unsigned ep;
+  uint64_t w[MB][W];
+  __device__ __forceinline__ void load() {
+#pragma unroll
+    for (int m = 0; m < MB; ++m)
+      if (col[m] >= 0) {
+        if constexpr (W == 2)
+          ld_words(z + (int64_t)col[m] * 2, w[m][0], w[m][1]);
+        else
+          w[m][0] = ld_word(z + col[m]);
+      }
   }
-  c.end(a, ok);
+  __device__ __forceinline__ void poll() { load(); }
+  __device__ __forceinline__ bool ready() const {
+    bool all = true;
+#pragma unroll
+    for (int m = 0; m < MB; ++m) {
+#pragma unroll
+      for (int k = 0; k < W; ++k) all = all && (col[m] < 0 || packet_is(w[m][k], ep));
+    }
+    return all;
+  }
+  __device__ __forceinline__ void finish() {
+    warp_wait(fail, [&] {
+      if (ready()) return true;
+      load();
+      return ready();
+    });
+  }
+  __device__ __forceinline__ T value(int m) const {
+    if constexpr (W == 2)
+      return packet_double(w[m][0], w[m][1]);
+    else
+      return __uint_as_float((unsigned)w[m][0]);
+  }
+};
+
+// The same for uniform blocks with at most kRowBlocks blocks per row.  What travels is z: every CTA keeps the p of the
+// columns that it needs (one thread per element, in shared memory for the product) and forms p = z + beta p itself,
+// the owner's expression on the owner's values.  So z is on its way together with the sums that give beta, an iteration
+// waits twice instead of three times, and an element is fetched once per block row instead of by each of its threads.
+// 64^2 p = 2 FP64 6.6 us per iteration, 7.3 with three waits; 24^3 p = 0 7.1 against 8.0.
+// No z is overwritten before everybody has it: the z of the next epoch is stored after the exchange of p.q, which every
+// CTA enters after its gather.
+template <class Rows>
+__global__ void __launch_bounds__(Rows::kT) pcg_gather_kernel(Rows rows, PcgCall<typename Rows::Value> a,
+                                                              uint64_t* __restrict__ packets,
+                                                              unsigned int* __restrict__ state) {
+  using T = typename Rows::Value;
+  constexpr int TH = Rows::kT, V = Rows::kV, SPLIT = Rows::kSplit, NP = Rows::kNP;
+  constexpr int MB = kRowBlocks / SPLIT;
+  constexpr int WPV = sizeof(T) / 4;
+  __shared__ T sm[TH];
+  __shared__ __align__(16) T ps[TH * MB];  // [block row of the CTA][block of the row][NP]
+  __shared__ double red[TH / 32][2];
+  if (!a.start && a.s[7] != kPcgRunning) return;
+  uint64_t* const pq_packets = packets;                           // 2 words per CTA
+  uint64_t* const rz_packets = packets + 2 * (int64_t)gridDim.x;  // 4 words per CTA
+  uint64_t* const z_packets = packets + 6 * (int64_t)gridDim.x;
+  unsigned int* const fail = state + 1;
+  unsigned ep = state[0];
+  bool ok = true;
+  CgScalars c{};
+  T vx = 0, vr = 0, vz = 0, vp = 0;
+  rows.begin();
+  rows.at(blockIdx.x);
+  T pe[MB];
+  Gather<T, MB> in;
+  in.z = z_packets;
+  in.fail = fail;
+#pragma unroll
+  for (int m = 0; m < MB; ++m) {
+    pe[m] = 0;
+    in.col[m] = -1;
+    for (int k = 0; k < WPV; ++k) in.w[m][k] = 0;
+  }
+  if (rows.valid) {
+    const int64_t k0 = rows.rp[rows.i] + rows.s, k1 = rows.rp[rows.i + 1];
+#pragma unroll
+    for (int m = 0; m < MB; ++m)
+      if (k0 + m * SPLIT < k1) in.col[m] = rows.ci[k0 + m * SPLIT] * NP + rows.r;
+  }
+  if (a.start) {
+    T ax = 0;
+    if (!a.zero) ax = rows.product(PlainVec<T, V>{a.x}, sm);
+    if (rows.own) {
+      vx = a.zero ? T(0) : __ldcg(a.x + rows.g);
+      vr = a.zero ? a.b[rows.g] : a.b[rows.g] - ax;
+    }
+    vz = a.dinv ? rows.solve(a.dinv, vr, sm) : vr;
+    vp = vz;
+    in.ep = ++ep;
+    double acc[2] = {0.0, 0.0}, tot[2];
+    if (rows.own) {
+      put_packet(z_packets + rows.g * WPV, vz, ep);
+      acc[0] = (double)vr * (double)vz;
+      acc[1] = (double)vr * (double)vr;
+    }
+    ok = exchange_sums<2, TH>(acc, tot, rz_packets, ep, fail, red, in);
+    c.begin(a, tot[0], tot[1]);
+#pragma unroll
+    for (int m = 0; m < MB; ++m) pe[m] = in.value(m);
+  } else {
+    c.resume(a);
+    if (rows.own) {
+      vx = __ldcg(a.x + rows.g);
+      vr = __ldcg(a.r + rows.g);
+      vz = __ldcg(a.z + rows.g);
+      vp = __ldcg(a.p + rows.g);
+    }
+#pragma unroll
+    for (int m = 0; m < MB; ++m)
+      if (in.col[m] >= 0) pe[m] = __ldcg(a.p + in.col[m]);
+  }
+  for (int n = 0; ok && !c.stop && n < a.cap; ++n) {
+#pragma unroll
+    for (int m = 0; m < MB; ++m)
+      if (in.col[m] >= 0) ps[rows.slot(rows.s + m * SPLIT) + rows.r] = pe[m];
+    sync_threads<TH>();
+    const T vq = rows.product(SlotVec<T, V>{ps}, sm);
+    {
+      double acc[1] = {rows.own ? (double)vp * (double)vq : 0.0}, tot[1];
+      ok = exchange_sums<1, TH>(acc, tot, pq_packets, ep, fail, red);
+      if (!ok) break;
+      c.pq = tot[0];
+    }
+    in.ep = ++ep;
+    {
+      const double alpha = c.rz / c.pq;
+      double acc[2] = {0.0, 0.0}, tot[2];
+      if (rows.own) {
+        vx = (T)((double)vx + alpha * (double)vp);
+        vr = (T)((double)vr - alpha * (double)vq);
+      }
+      vz = a.dinv ? rows.solve(a.dinv, vr, sm) : vr;
+      if (rows.own) {
+        put_packet(z_packets + rows.g * WPV, vz, ep);
+        acc[0] = (double)vr * (double)vz;
+        acc[1] = (double)vr * (double)vr;
+      }
+      ok = exchange_sums<2, TH>(acc, tot, rz_packets, ep, fail, red, in);
+      if (!ok) break;
+      c.step(a, tot[0], tot[1]);
+    }
+    if (c.stop) break;
+    vp = (T)((double)vz + c.beta * (double)vp);
+#pragma unroll
+    for (int m = 0; m < MB; ++m) pe[m] = (T)((double)in.value(m) + c.beta * (double)pe[m]);
+  }
+  if (rows.own) {
+    a.x[rows.g] = vx;
+    if (!c.stop) {
+      a.r[rows.g] = vr;
+      a.z[rows.g] = vz;
+      a.p[rows.g] = vp;
+    }
+  }
+  small_end(a, c, ok, ep, state);
 }
 
 // ---- choice and launch ------------------------------------------------------------------------------------------
@@ -846,9 +1085,9 @@ template <typename T, typename ST, class F>
 bool pick_large(const Matrix& A, F&& f) {
   if (pick_uniform<T, ST>(A, [&](auto np, auto v) {
         constexpr int NP = decltype(np)::value, V = decltype(v)::value;
-        // Few and large CTAs: a barrier takes as long as its arrivals (32^3 p = 1 FP64 15.2 us per iteration with two CTAs
-        // of 512 threads per SM, 17.2 with four of 256).  64 registers per thread; blocks of 10 stream better with 48 and
-        // more threads.
+        // Few and large CTAs: a barrier takes as long as its arrivals (32^3 p = 1 FP64 15.2 us per iteration with two
+        // CTAs of 512 threads per SM, 17.2 with four of 256).  64 registers per thread; blocks of 10 stream better with
+        // 48 and more threads.
         constexpr int THREADS = NP == 10 ? 640 : 512;
         return f(Tag<UniformRows<T, NP, V, 1, ST, THREADS, 2>>{});
       }))
@@ -910,6 +1149,14 @@ void cooperative(const void* kernel, int grid, int threads, size_t smem, void** 
   BSGPU_CHECK_LAUNCH();
 }
 
+template <class Rows>
+const void* small_kernel(bool gather) {
+  if constexpr (Rows::kGathers) {
+    if (gather) return reinterpret_cast<const void*>(&pcg_gather_kernel<Rows>);
+  }
+  return reinterpret_cast<const void*>(&pcg_small_kernel<Rows>);
+}
+
 template <typename T, typename ST>
 void run_impl(PcgLaunch& l, const ST* vals, const PcgCall<T>& c, cudaStream_t st) {
   const Matrix& A = *l.A;
@@ -923,7 +1170,7 @@ void run_impl(PcgLaunch& l, const ST* vals, const PcgCall<T>& c, cudaStream_t st
       using Rows = typename decltype(tag)::Rows;
       Rows rows = rows_of<Rows>(A, vals);
       void* args[4] = {&rows, &call, &packets, &bar};
-      cooperative(reinterpret_cast<const void*>(&pcg_small_kernel<Rows>), l.grid, Rows::kT, 0, args, st);
+      cooperative(small_kernel<Rows>(l.gather), l.grid, Rows::kT, 0, args, st);
       return true;
     });
   } else {
@@ -943,12 +1190,15 @@ void run_impl(PcgLaunch& l, const ST* vals, const PcgCall<T>& c, cudaStream_t st
 template <typename T, typename ST>
 bool init_small(PcgLaunch& l, cudaStream_t st) {
   const Matrix& A = *l.A;
+  int64_t most = 0;
+  for (int64_t i = 0; i < A.nb; ++i) most = std::max(most, A.h_rp[i + 1] - A.h_rp[i]);
+  l.gather = most <= kRowBlocks;
   for (int w : {4, 2, 1}) {
     const bool ok = pick_small<T, ST>(A, w, [&](auto tag) {
       using Rows = typename decltype(tag)::Rows;
       int64_t tiles = A.ncta;
       if constexpr (!IsGeneral<Rows>::value) tiles = (A.nb + Rows::BPC - 1) / Rows::BPC;
-      if (tiles > resident(reinterpret_cast<const void*>(&pcg_small_kernel<Rows>), Rows::kT, 0)) return false;
+      if (tiles > resident(small_kernel<Rows>(l.gather), Rows::kT, 0)) return false;
       l.grid = (int)tiles;
       return true;
     });
@@ -963,7 +1213,7 @@ bool init_small(PcgLaunch& l, cudaStream_t st) {
 }
 
 // The large kernel, up to the sizes at which the separate launches' products (full occupancy) weigh more than what the
-// one launch saves: 24^3 p = 3 FP64 (299 MB) 74 us per iteration against 78, 31^3 (649 MB) 177 against 160; with
+// one launch saves: 24^3 p = 3 FP64 (299 MB) 71 us per iteration against 78, 31^3 (649 MB) 177 against 160; with
 // blocks of 10, 64^3 p = 2 (1.45 GB) 369 against 367.
 template <typename T, typename ST>
 bool init_large(PcgLaunch& l) {

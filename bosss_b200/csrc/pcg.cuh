@@ -27,6 +27,7 @@ struct PcgLaunch {
   int split = 1;              // kSmall: threads per DOF row
   DBuf<unsigned char> r2;     // kLarge: the second residual buffer
   DBuf<double> partial;       // kLarge: sums per CTA [2 * grid]
+  bool gather = false;        // kSmall: rows short enough for the form that gathers its operand per CTA
   DBuf<uint64_t> packets;     // kSmall: p.q [2 * grid], r.z and r.r [4 * grid], the direction [N or 2 N]
   DBuf<unsigned int> bar;     // arrivals (or the epoch of the packets), failure, exits
   // false: the matrix is served by separate launches (too large, or no kernel for its layout)

@@ -8,13 +8,14 @@ import scipy.sparse as sp
 pytestmark = pytest.mark.gpu
 
 
-def _system(Np, nb, two, seed):
-    """Symmetric diagonally dominant block system on a ring with two further neighbours per row."""
+def _system(Np, nb, two, seed, far=()):
+    """Symmetric diagonally dominant block system on a ring with two further neighbours per row and those at `far`."""
     rng = np.random.default_rng(seed)
     nspc = 1 + (rng.random(nb) < 0.3).astype(np.int32) if two else np.ones(nb, np.int32)
     L = nspc.astype(np.int64) * Np
     hop = max(2, int(round(nb ** 0.5)))
-    pairs = {(min(i, j), max(i, j)) for i in range(nb) for j in ((i + 1) % nb, (i + hop) % nb) if i != j}
+    pairs = {(min(i, j), max(i, j)) for i in range(nb) for j in {(i + d) % nb for d in (1, hop, *far)}
+             if i != j}
     blocks = {}
     for i, j in pairs:
         v = rng.standard_normal((L[i], L[j])) * (0.1 / np.sqrt(Np))
@@ -62,8 +63,20 @@ def _cg(A, D, x, b, steps):
     (15, 6000, False, True), (20, 7, False, True), (20, 4500, False, True), (7, 300, False, True),
     (9, 12000, False, True), (1, 700, True, True), (10, 300, True, True), (4, 30000, True, False)])
 def test_cg_steps(cuda, Np, nb, two, precond):
+    _check_steps(Np, nb, two, precond)
+
+
+# the operand gathered once per CTA: rows of 8 blocks at most (7 and 9 here), four or two threads per DOF row
+@pytest.mark.parametrize("Np,nb,far", [
+    (1, 900, (7,)), (1, 900, (7, 11)), (6, 300, (7,)), (6, 300, (7, 11)), (3, 8000, (7,)), (10, 3000, (7,)),
+    (10, 3000, (7, 11)), (15, 2000, (7,)), (20, 1500, (7,)), (20, 200, (7,)), (4, 18000, (7,))])
+def test_cg_row_lengths(cuda, Np, nb, far):
+    _check_steps(Np, nb, False, True, far)
+
+
+def _check_steps(Np, nb, two, precond, far=()):
     from bosss_b200.solvers import BlockMsrMatrix, MultigridOperator, SoftPCGConfig
-    rp, ci, values, nspc, A, D = _system(Np, nb, two, 100 * Np + nb)
+    rp, ci, values, nspc, A, D = _system(Np, nb, two, 100 * Np + nb, far)
     rng = np.random.default_rng(5)
     N = A.shape[0]
     b, x0 = rng.standard_normal(N), rng.standard_normal(N)
