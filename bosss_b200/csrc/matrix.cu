@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(256) spmv_general_kernel(
 // sub-blocks of NP columns, each streamed with the fully unrolled chunk loop of the uniform kernel (V divides NP,
 // so no chunk straddles a species boundary and there is no scalar tail).  SPLIT threads share a row, each with every
 // SPLIT-th block (small systems, see launch_typed): their sums meet in shared memory.
-template <typename T, int NP, int NS, int V, int MODE, int SPLIT>
+template <typename T, int NP, int NS, int V, int MODE, int SPLIT, bool AHEAD>
 __device__ __forceinline__ void typed_rows(int BPC, int64_t b0, int64_t nrows, const int32_t* __restrict__ rows,
                                            const int64_t* __restrict__ rp, const int32_t* __restrict__ ci,
                                            const int32_t* __restrict__ len, const int64_t* __restrict__ i0,
@@ -318,7 +318,7 @@ __device__ __forceinline__ void typed_rows(int BPC, int64_t b0, int64_t nrows, c
         }
       }
     };
-    if constexpr (sizeof(T) == 4) {
+    if constexpr (AHEAD) {
       // Two steps ahead the next block's column, one step ahead what hangs on it, so that a block's chain of lookups
       // (column, then length and offsets) is over when its turn comes: 40^3 p = 2 FP32 (190 MB) 60 us, 72 with the
       // lookups in place; with FP64 blocks, twice as long each, the plain loop is the faster one (84 against 89 us).
@@ -396,7 +396,7 @@ __device__ __forceinline__ void typed_rows(int BPC, int64_t b0, int64_t nrows, c
 }
 
 // One launch for both species counts: CTAs [0, cta1) take the one-species rows, the rest the two-species rows.
-template <typename T, int NP, int V, int MODE, int SPLIT>
+template <typename T, int NP, int V, int MODE, int SPLIT, bool AHEAD>
 __global__ void __launch_bounds__(256) spmv_typed_kernel(
     const int64_t* __restrict__ rp, const int32_t* __restrict__ ci, const int32_t* __restrict__ len,
     const int64_t* __restrict__ i0, const int64_t* __restrict__ boff, const int32_t* __restrict__ rows,
@@ -406,11 +406,11 @@ __global__ void __launch_bounds__(256) spmv_typed_kernel(
   if (active != nullptr && *active == 0) return;
   const int bpc1 = blockDim.x / (NP * SPLIT), bpc2 = blockDim.x / (2 * NP * SPLIT);
   if ((int64_t)blockIdx.x < cta1)
-    typed_rows<T, NP, 1, V, MODE, SPLIT>(bpc1, (int64_t)blockIdx.x * bpc1, n1, rows, rp, ci, len, i0, boff, vals, x, z,
-                                         y, alpha, beta, dinv, doff);
+    typed_rows<T, NP, 1, V, MODE, SPLIT, AHEAD>(bpc1, (int64_t)blockIdx.x * bpc1, n1, rows, rp, ci, len, i0, boff,
+                                                vals, x, z, y, alpha, beta, dinv, doff);
   else
-    typed_rows<T, NP, 2, V, MODE, SPLIT>(bpc2, ((int64_t)blockIdx.x - cta1) * bpc2, n2, rows + n1, rp, ci, len, i0,
-                                         boff, vals, x, z, y, alpha, beta, dinv, doff);
+    typed_rows<T, NP, 2, V, MODE, SPLIT, AHEAD>(bpc2, ((int64_t)blockIdx.x - cta1) * bpc2, n2, rows + n1, rp, ci, len,
+                                                i0, boff, vals, x, z, y, alpha, beta, dinv, doff);
 }
 
 // y = alpha * Dinv * b for uniform blocks of NP (column-major blocks): one thread per DOF row, the block row's NP columns
@@ -630,7 +630,14 @@ void launch_typed_split(const Matrix& A, const T* vals, const T* x, const T* z, 
   const int64_t bpc1 = threads / (NP * SPLIT), bpc2 = threads / (2 * NP * SPLIT);
   const int64_t cta1 = (A.grp_n1 + bpc1 - 1) / bpc1, cta2 = (A.grp_n2 + bpc2 - 1) / bpc2;
   if (cta1 + cta2 == 0) return;
-  spmv_typed_kernel<T, NP, V, MODE, SPLIT><<<(unsigned)(cta1 + cta2), threads, 0, st>>>(
+  auto kernel = &spmv_typed_kernel<T, NP, V, MODE, SPLIT, sizeof(T) == 4>;
+  // The lookups ahead cost blocks of 10 eight registers and with them a quarter of the threads, which long products
+  // want more: 40^3 p = 2 (640,000 rows) 60 us against 72 with the plain loop, 60^3 p = 2 143 against 148, 500 x 600
+  // p = 3 (3.1 million rows) 139.8 against 140.0, 573 x 761 p = 3 213 against 208, 800^2 p = 3 320 against 303.
+  if constexpr (sizeof(T) == 4 && NP == 10 && MODE == 0 && SPLIT == 1) {
+    if (A.N > 3000000) kernel = &spmv_typed_kernel<T, NP, V, MODE, SPLIT, false>;
+  }
+  kernel<<<(unsigned)(cta1 + cta2), threads, 0, st>>>(
       A.rp.p, A.ci.p, A.len.p, A.i0.p, A.boff.p, A.grp_rows.p, A.grp_n1, A.grp_n2, cta1, vals, x, z, y, alpha, beta,
       dinv, doff, active);
   BSGPU_CHECK_LAUNCH();
